@@ -4,9 +4,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 
 #include "hx_common.cuh"
@@ -78,29 +80,64 @@ static inline float bf16_bits_to_f32(uint16_t b) {
 }
 
 // ------------------------------------------------------------------------------------------ DeviceTensor
-Result<DeviceTensor> DeviceTensor::empty(const Shape &shape, DType dtype, const Device &device) {
+// Owns one device block; a pooled one returns to the block cache unless its address was given to a caller.
+struct DeviceTensor::Storage {
+    void *p = nullptr;
+    int dev = 0;
+    bool pooled = false;
+    std::atomic<bool> escaped{false};
+    ~Storage() {
+        if (pooled && !escaped.load(std::memory_order_acquire)) hx::pool_release(p, dev);
+        else hx::pool_discard(p, dev);
+    }
+};
+
+static Result<Unit> check_shape(const Shape &shape, const Device &device) {
     for (auto d : shape.as_slice())
         if (d < 0) return err(HX_ERR_INVALID_DIMENSION, "negative dimension in shape " + shape_str(shape));
-    HELIX_TRY(use_device(device));
+    return use_device(device);
+}
+
+Result<DeviceTensor> DeviceTensor::empty(const Shape &shape, DType dtype, const Device &device) {
+    HELIX_TRY(check_shape(shape, device));
     DeviceTensor t;
     t.shape_ = shape;
     t.dtype_ = dtype;
     t.device_ = device;
     const size_t bytes = (size_t)shape.numel() * dtype_size(dtype);
     if (bytes > 0) {
-        void *p = nullptr;
-        HELIX_TRY_ABI(hx_alloc(&p, bytes));
-        const int dev = device.id;
-        t.storage_ = std::shared_ptr<void>(p, [dev](void *q) {
-            int cur = 0;
-            cudaGetDevice(&cur);
-            if (cur != dev) cudaSetDevice(dev);
-            cudaFree(q);
-            if (cur != dev) cudaSetDevice(cur);
-        });
-        t.ptr_ = p;
+        auto st = std::make_shared<Storage>();
+        HELIX_TRY_ABI(hx_alloc(&st->p, bytes));
+        st->dev = device.id;
+        t.ptr_ = st->p;
+        t.storage_ = std::move(st);
     }
     return t;
+}
+
+Result<DeviceTensor> DeviceTensor::pooled(const Shape &shape, DType dtype, const Device &device) {
+    HELIX_TRY(check_shape(shape, device));
+    DeviceTensor t;
+    t.shape_ = shape;
+    t.dtype_ = dtype;
+    t.device_ = device;
+    const size_t bytes = (size_t)shape.numel() * dtype_size(dtype);
+    if (bytes > 0) {
+        auto st = std::make_shared<Storage>();
+        HELIX_TRY_ABI(hx::pool_alloc(&st->p, bytes));
+        st->dev = device.id;
+        st->pooled = true;
+        t.ptr_ = st->p;
+        t.storage_ = std::move(st);
+    }
+    return t;
+}
+
+void *DeviceTensor::data_for_caller() const {
+    if (storage_ && storage_->pooled && !storage_->escaped.exchange(true, std::memory_order_acq_rel)) {
+        if (use_device(device_).ok()) cudaStreamSynchronize(nullptr);
+    }
+    return ptr_;
 }
 
 Result<DeviceTensor> DeviceTensor::zeros(const Shape &shape, DType dtype, const Device &device) {
@@ -109,6 +146,19 @@ Result<DeviceTensor> DeviceTensor::zeros(const Shape &shape, DType dtype, const 
     if (r.value().numel() > 0)
         HELIX_TRY_ABI(hx_memset(r.value().data(), 0, (size_t)r.value().numel() * dtype_size(dtype), nullptr));
     return r;
+}
+
+// An upload need not be waited for when the tensor is only used in stream order (pooled and not given to a caller; a
+// module's parameters may be read from any stream) and the source is ordinary host memory, all of which a copy has read
+// when the call returns.  (Pinned memory is read later, in stream order.)
+bool DeviceTensor::may_return_early(const void *host) const {
+    if (!storage_ || !storage_->pooled || storage_->escaped.load(std::memory_order_acquire)) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 Result<Unit> DeviceTensor::copy_from_host_f32(const float *data, int64_t n) {
@@ -123,28 +173,31 @@ Result<Unit> DeviceTensor::copy_from_host_f32(const float *data, int64_t n) {
         std::vector<uint16_t> tmp((size_t)n);
         for (int64_t i = 0; i < n; ++i) tmp[(size_t)i] = f32_to_bf16_bits(data[i]);
         HELIX_TRY_ABI(hx_memcpy_h2d(ptr_, tmp.data(), (size_t)n * 2, nullptr));
+        if (may_return_early(tmp.data())) return Unit{};
         HELIX_TRY_ABI(hx_stream_synchronize(nullptr));  // tmp dies at scope end
+        return Unit{};
     } else {
         return err(HX_ERR_DTYPE_MISMATCH, "copy_from_host_f32 into a U8 tensor");
     }
-    HELIX_TRY_ABI(hx_stream_synchronize(nullptr));
+    if (!may_return_early(data)) HELIX_TRY_ABI(hx_stream_synchronize(nullptr));
     return Unit{};
 }
 
-Result<DeviceTensor> DeviceTensor::from_host_f32(const float *data, const Shape &shape, DType dtype, const Device &device) {
-    auto r = empty(shape, dtype, device);
+Result<DeviceTensor> DeviceTensor::from_host_f32(const float *data, const Shape &shape, DType dtype, const Device &device,
+                                                  bool from_pool) {
+    auto r = from_pool ? pooled(shape, dtype, device) : empty(shape, dtype, device);
     if (!r.ok()) return r;
     HELIX_TRY(r.value().copy_from_host_f32(data, shape.numel()));
     return r;
 }
 
 Result<DeviceTensor> DeviceTensor::from_host_u8(const uint8_t *data, const Shape &shape, const Device &device) {
-    auto r = empty(shape, DType::U8, device);
+    auto r = pooled(shape, DType::U8, device);
     if (!r.ok()) return r;
     if (shape.numel() > 0) {
         if (!data) return err(HX_ERR_INVALID_INPUT, "from_host_u8: data is NULL");
         HELIX_TRY_ABI(hx_memcpy_h2d(r.value().data(), data, (size_t)shape.numel(), nullptr));
-        HELIX_TRY_ABI(hx_stream_synchronize(nullptr));
+        if (!r.value().may_return_early(data)) HELIX_TRY_ABI(hx_stream_synchronize(nullptr));
     }
     return r;
 }
@@ -172,7 +225,7 @@ Result<Unit> DeviceTensor::to_host_f32(float *out, int64_t n) const {
 }
 
 Result<DeviceTensor> DeviceTensor::clone() const {
-    auto r = empty(shape_, dtype_, device_);
+    auto r = pooled(shape_, dtype_, device_);
     if (!r.ok()) return r;
     const size_t bytes = (size_t)numel() * dtype_size(dtype_);
     if (bytes > 0) {
@@ -192,26 +245,26 @@ Result<DeviceTensor> DeviceTensor::reshape(const Shape &shape) const {
 
 // Normal(mean, std) / uniform / Bernoulli / constant initialisers (TensorRandom, crates/tensor-core/src/tensor.rs:212-233),
 // drawn on the host from the seeded counter streams above
-Result<DeviceTensor> init_normal(const Shape &shape, double stddev, DType dtype, const Device &device, double mean) {
+Result<DeviceTensor> init_normal(const Shape &shape, double stddev, DType dtype, const Device &device, double mean, bool from_pool) {
     if (shape.numel() < 0) return err(HX_ERR_INVALID_DIMENSION, "negative dimension in shape " + shape_str(shape));
     std::vector<float> h((size_t)shape.numel());
     Rng rng;
     for (auto &v : h) v = (float)(mean + stddev * rng.normal());
-    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device);
+    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device, from_pool);
 }
-Result<DeviceTensor> init_uniform(const Shape &shape, double lo, double hi, DType dtype, const Device &device) {
+Result<DeviceTensor> init_uniform(const Shape &shape, double lo, double hi, DType dtype, const Device &device, bool from_pool) {
     if (shape.numel() < 0) return err(HX_ERR_INVALID_DIMENSION, "negative dimension in shape " + shape_str(shape));
     std::vector<float> h((size_t)shape.numel());
     Rng rng;
     for (auto &v : h) v = (float)(lo + (hi - lo) * rng.uniform01());
-    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device);
+    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device, from_pool);
 }
-Result<DeviceTensor> init_bernoulli(const Shape &shape, double p, DType dtype, const Device &device) {
+Result<DeviceTensor> init_bernoulli(const Shape &shape, double p, DType dtype, const Device &device, bool from_pool) {
     if (shape.numel() < 0) return err(HX_ERR_INVALID_DIMENSION, "negative dimension in shape " + shape_str(shape));
     std::vector<float> h((size_t)shape.numel());
     Rng rng;
     for (auto &v : h) v = rng.uniform01() < p ? 1.f : 0.f;
-    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device);
+    return DeviceTensor::from_host_f32(h.data(), shape, dtype, device, from_pool);
 }
 static Result<DeviceTensor> init_const(const Shape &shape, float value, DType dtype, const Device &device) {
     std::vector<float> h((size_t)shape.numel(), value);
@@ -256,7 +309,7 @@ Result<DeviceTensor> Linear::forward(const DeviceTensor &x) const {
     std::vector<int64_t> od = x.shape().as_slice();
     od.back() = out_f;
     DeviceTensor y;
-    HELIX_ASSIGN(y, DeviceTensor::empty(Shape(od), x.dtype(), device_));
+    HELIX_ASSIGN(y, DeviceTensor::pooled(Shape(od), x.dtype(), device_));
     const float *b = has_bias ? static_cast<const float *>(bias.data()) : nullptr;
     if (x.dtype() == DType::BF16 && in_f % 8 == 0)
         HELIX_TRY_ABI(hx_gemm_bf16(x.data(), in_f, weight.data(), in_f, b, y.data(), out_f, HX_BF16, (int)rows, (int)out_f,
@@ -290,7 +343,7 @@ Result<DeviceTensor> RMSNorm::forward(const DeviceTensor &x) const {
     HELIX_TRY(rows_of(x, d, "RMSNorm", &rows));
     if (x.dtype() == DType::U8) return err(HX_ERR_DTYPE_MISMATCH, "RMSNorm: U8 input");
     DeviceTensor y;
-    HELIX_ASSIGN(y, DeviceTensor::empty(x.shape(), x.dtype(), device_));
+    HELIX_ASSIGN(y, DeviceTensor::pooled(x.shape(), x.dtype(), device_));
     HELIX_TRY_ABI(hx_rmsnorm_fwd(x.data(), (int)x.dtype(), nullptr, static_cast<const float *>(weight.data()), y.data(),
                                  (int)x.dtype(), rows, (int)d, eps, nullptr));
     return y;
@@ -337,13 +390,12 @@ Result<DeviceTensor> S4Block::forward_ssm(const DeviceTensor &u) const {
     // the reference labels the result [d_model, L] although its buffer is time-major; here the shape says what
     // the buffer holds: [L, d_model]
     DeviceTensor y, ws;
-    HELIX_ASSIGN(y, DeviceTensor::empty(Shape({L, d_model}), DType::F32, device_));
+    HELIX_ASSIGN(y, DeviceTensor::pooled(Shape({L, d_model}), DType::F32, device_));
     const size_t wb = hx_s4_ref_workspace_bytes((int)L, (int)d_state);
-    HELIX_ASSIGN(ws, DeviceTensor::empty(Shape({(int64_t)wb}), DType::U8, device_));
+    HELIX_ASSIGN(ws, DeviceTensor::pooled(Shape({(int64_t)wb}), DType::U8, device_));
     auto f = [](const DeviceTensor &t) { return static_cast<const float *>(t.data()); };
     HELIX_TRY_ABI(hx_s4_ref_forward_ssm(f(u), f(A_real), f(A_imag), f(B), f(C), f(D), 0.1f, static_cast<float *>(y.data()),
                                         (int)d_model, (int)L, (int)d_state, ws.data(), wb, nullptr));
-    HELIX_TRY_ABI(hx_stream_synchronize(nullptr));  // ws is released on return
     return y;
 }
 
@@ -353,7 +405,7 @@ Result<DeviceTensor> S4Block::forward(const DeviceTensor &u) const {
     if (u.dtype() == DType::U8) return err(HX_ERR_DTYPE_MISMATCH, "S4Block: U8 input");
     const int64_t L = u.shape().dim(u.ndim() - 2), Bsz = rows / L;
     DeviceTensor y;
-    HELIX_ASSIGN(y, DeviceTensor::empty(u.shape(), u.dtype(), device_));
+    HELIX_ASSIGN(y, DeviceTensor::pooled(u.shape(), u.dtype(), device_));
     auto f = [](const DeviceTensor &t) { return static_cast<const float *>(t.data()); };
     HELIX_TRY_ABI(hx_s4_diag_fwd(u.data(), f(A_diag), f(B_diag), f(C_diag), f(delta), f(D), y.data(), (int)Bsz, (int)L,
                                  (int)d_model, (int)d_state, (int)u.dtype(), nullptr));
@@ -494,12 +546,11 @@ Result<DeviceTensor> MambaBlock::forward(const DeviceTensor &x) const {
     const int64_t L = x.shape().dim(x.ndim() - 2), Bsz = rows / L;
     HELIX_TRY(use_device(device_));
     DeviceTensor y, ws;
-    HELIX_ASSIGN(y, DeviceTensor::empty(x.shape(), dtype, device_));
+    HELIX_ASSIGN(y, DeviceTensor::pooled(x.shape(), dtype, device_));
     if (rows == 0) return y;
     const size_t wb = workspace_bytes(Bsz, L);
-    HELIX_ASSIGN(ws, DeviceTensor::empty(Shape({(int64_t)wb}), DType::U8, device_));
-    HELIX_TRY(forward_into(x.data(), y.data(), Bsz, L, ws.data(), wb, nullptr));
-    HELIX_TRY_ABI(hx_stream_synchronize(nullptr));  // the workspace is released on return
+    HELIX_ASSIGN(ws, DeviceTensor::pooled(Shape({(int64_t)wb}), DType::U8, device_));
+    HELIX_TRY(forward_into(x.data(), y.data(), Bsz, L, ws.data(), wb, nullptr));  // ws returns to the cache in stream order
     return y;
 }
 std::vector<const DeviceTensor *> MambaBlock::parameters() const {
@@ -540,7 +591,9 @@ Result<Unit> Sequential::parameters_updated() {
 
 // ------------------------------------------------------------------------------------------ ByteLM
 struct ByteLM::Buffers {
-    int64_t batch = 0, seq_len = 0;
+    int64_t batch = 0, seq_len = 0;  // shape of the last call
+    int64_t tokens_cap = 0;          // batch * seq_len the buffers hold
+    size_t workspace_cap = 0;
     DeviceTensor tokens, resid, normed, block_out, logits, workspace;
 };
 
@@ -548,16 +601,23 @@ struct ByteLM::Buffers {
 // captured graph of one step over those buffers.
 struct ByteLM::Decode {
     int64_t batch = 0;
+    int64_t cap = 0;                    // batch the buffers hold; a smaller batch uses their front
     std::vector<DeviceTensor> h, conv;  // per layer: [B, E, N] fp32, [B, 3, E] model dtype
     DeviceTensor tokens, resid, normed, block_out, logits, workspace;
     cudaStream_t capture_stream = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    std::map<int64_t, cudaGraphExec_t> execs;  // by batch
     int64_t steps = 0;
+    void drop_graphs() {
+        for (auto &e : execs) cudaGraphExecDestroy(e.second);
+        execs.clear();
+    }
     ~Decode() {
-        if (exec) cudaGraphExecDestroy(exec);
+        drop_graphs();
         if (capture_stream) cudaStreamDestroy(capture_stream);
     }
 };
+static constexpr size_t kDecodeGraphs = 8;    // batch sizes whose step stays captured
+static constexpr size_t kForwardGraphs = 32;  // captured forwards kept (the lengths a queue of prompts repeats)
 
 // Event-based stage timing: per forward, events[0] before the embedding, then per layer one event before the
 // norm and the block's seven, then events before the final norm, before the head and after it.
@@ -681,18 +741,52 @@ Result<Unit> ByteLM::parameters_updated() {
     return Unit{};
 }
 
-Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len) {
-    if (buf_ && buf_->batch == batch && buf_->seq_len == seq_len) return Unit{};
-    delete buf_;
-    buf_ = new Buffers();
+// Makes the activation buffers hold (batch, seq_len).  They only ever grow, by at least half of what they are: prompts of
+// changing length run in the same memory (allocating per shape cost 1 to 100 ms a prompt, and every captured forward with
+// it, since cudaFree waits for the device).  `moved` tells that captured forwards point into memory that is gone.
+Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len, bool *moved) {
+    if (moved) *moved = false;
     const int64_t T = batch * seq_len;
-    HELIX_ASSIGN(buf_->tokens, DeviceTensor::empty(Shape({T}), DType::U8, device_));
-    HELIX_ASSIGN(buf_->resid, DeviceTensor::empty(Shape({T, d_model}), DType::F32, device_));
-    HELIX_ASSIGN(buf_->normed, DeviceTensor::empty(Shape({T, d_model}), dtype, device_));
-    HELIX_ASSIGN(buf_->block_out, DeviceTensor::empty(Shape({T, d_model}), dtype, device_));
-    HELIX_ASSIGN(buf_->logits, DeviceTensor::empty(Shape({T, 256}), dtype, device_));
+    if (!buf_) buf_ = new Buffers();
+    if (T > buf_->tokens_cap) {
+        if (moved) *moved = true;
+        const int64_t grown = buf_->tokens_cap + buf_->tokens_cap / 2;
+        const int64_t cap = T > grown ? T : grown;
+        delete buf_;
+        buf_ = new Buffers();
+        auto fill = [&](int64_t n) -> Result<Unit> {
+            HELIX_ASSIGN(buf_->tokens, DeviceTensor::empty(Shape({n}), DType::U8, device_));
+            HELIX_ASSIGN(buf_->resid, DeviceTensor::empty(Shape({n, d_model}), DType::F32, device_));
+            HELIX_ASSIGN(buf_->normed, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
+            HELIX_ASSIGN(buf_->block_out, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
+            HELIX_ASSIGN(buf_->logits, DeviceTensor::empty(Shape({n, 256}), dtype, device_));
+            buf_->tokens_cap = n;
+            return Unit{};
+        };
+        auto r = fill(cap);
+        if (!r.ok() && cap > T) {  // no room for the spare half
+            delete buf_;
+            buf_ = new Buffers();
+            r = fill(T);
+        }
+        if (!r.ok()) {
+            delete buf_;
+            buf_ = nullptr;
+            return r.error();
+        }
+    }
     const size_t wb = blocks[0]->workspace_bytes(batch, seq_len);
-    HELIX_ASSIGN(buf_->workspace, DeviceTensor::empty(Shape({(int64_t)wb}), DType::U8, device_));
+    if (wb > buf_->workspace_cap) {
+        if (moved) *moved = true;
+        const size_t cap = std::max(wb, buf_->workspace_cap + buf_->workspace_cap / 2);
+        buf_->workspace_cap = 0;
+        buf_->workspace = DeviceTensor();
+        auto w = DeviceTensor::empty(Shape({(int64_t)cap}), DType::U8, device_);
+        if (!w.ok() && cap > wb) w = DeviceTensor::empty(Shape({(int64_t)wb}), DType::U8, device_);
+        if (!w.ok()) return w.error();
+        buf_->workspace = std::move(w.value());
+        buf_->workspace_cap = (size_t)buf_->workspace.numel();
+    }
     buf_->batch = batch;
     buf_->seq_len = seq_len;
     return Unit{};
@@ -717,8 +811,14 @@ Result<Unit> ByteLM::prefill_device(const uint8_t *tokens_dev, void *logits_dev,
     return run_layers(tokens_dev, logits_dev, batch, seq_len, stream, true);
 }
 
-Result<Unit> ByteLM::ensure_decode(int64_t batch) {
-    if (dec_ && dec_->batch == batch) return Unit{};
+// The decode state of `batch` sequences.  The buffers grow only; `moved` as for ensure_buffers.
+Result<Unit> ByteLM::ensure_decode(int64_t batch, bool *moved) {
+    if (moved) *moved = false;
+    if (dec_ && dec_->cap >= batch) {
+        dec_->batch = batch;
+        return Unit{};
+    }
+    if (moved) *moved = true;
     delete dec_;
     dec_ = new Decode();
     const MambaBlock &b0 = *blocks[0];
@@ -736,6 +836,7 @@ Result<Unit> ByteLM::ensure_decode(int64_t batch) {
     HELIX_ASSIGN(dec_->logits, DeviceTensor::empty(Shape({batch, 256}), dtype, device_));
     HELIX_ASSIGN(dec_->workspace, DeviceTensor::empty(Shape({(int64_t)b0.step_workspace_bytes(batch)}), DType::U8, device_));
     dec_->batch = batch;
+    dec_->cap = batch;
     return Unit{};
 }
 
@@ -783,7 +884,8 @@ Result<Unit> ByteLM::decode_step_device(const uint8_t *tokens_dev, void *logits_
         return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: token copy failed");
     // The first step runs as plain launches (it also sets the kernels' attributes); the second one is captured
     // on a private stream (capture is not allowed on the legacy default stream) and every later step replays it.
-    if (decode_graph_ && dec_->steps >= 1 && !dec_->exec) {
+    auto it = dec_->execs.find(batch);
+    if (decode_graph_ && dec_->steps >= 1 && it == dec_->execs.end()) {
         if (!dec_->capture_stream && cudaStreamCreateWithFlags(&dec_->capture_stream, cudaStreamNonBlocking) != cudaSuccess)
             return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: cannot create the capture stream");
         if (cudaStreamBeginCapture(dec_->capture_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
@@ -796,15 +898,15 @@ Result<Unit> ByteLM::decode_step_device(const uint8_t *tokens_dev, void *logits_
             return r.error();
         }
         if (ce != cudaSuccess || !graph) return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: stream capture failed");
-        const cudaError_t ie = cudaGraphInstantiate(&dec_->exec, graph, 0);
+        cudaGraphExec_t exec = nullptr;
+        const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) {
-            dec_->exec = nullptr;
-            return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: cudaGraphInstantiate failed");
-        }
+        if (ie != cudaSuccess) return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: cudaGraphInstantiate failed");
+        if (dec_->execs.size() >= kDecodeGraphs) dec_->drop_graphs();
+        it = dec_->execs.emplace(batch, exec).first;
     }
-    if (decode_graph_ && dec_->exec) {
-        if (cudaGraphLaunch(dec_->exec, st) != cudaSuccess) return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: graph launch failed");
+    if (decode_graph_ && it != dec_->execs.end()) {
+        if (cudaGraphLaunch(it->second, st) != cudaSuccess) return err(HX_ERR_BACKEND, "ByteLM::decode_step_device: graph launch failed");
     } else {
         HELIX_TRY(enqueue_step(stream));
     }
@@ -820,17 +922,18 @@ Result<Unit> ByteLM::run_layers(const uint8_t *tokens_dev, void *logits_dev, int
     std::lock_guard<std::recursive_mutex> lock(mu_);
     if (batch <= 0 || seq_len <= 0) return err(HX_ERR_INVALID_DIMENSION, "ByteLM: batch and seq_len must be positive");
     HELIX_TRY(use_device(device_));
-    const bool had_buffers = buf_ && buf_->batch == batch && buf_->seq_len == seq_len;
-    HELIX_TRY(ensure_buffers(batch, seq_len));
-    if (!had_buffers && fwd_) fwd_->clear();  // the graphs point into the old activation buffers
+    bool moved = false;
+    auto eb = ensure_buffers(batch, seq_len, &moved);
+    if (moved && fwd_) fwd_->clear();  // the graphs point into the old activation buffers
+    if (!eb.ok()) return eb.error();
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing((cudaStream_t)stream, &cap);
     if (!forward_graph_ || prof_ || cap != cudaStreamCaptureStatusNone)
         return run_layers_plain(tokens_dev, logits_dev, batch, seq_len, stream, keep_state);
     if (keep_state) {
-        const bool had_decode = dec_ && dec_->batch == batch;
-        HELIX_TRY(ensure_decode(batch));  // allocate outside any capture
-        if (!had_decode && fwd_) fwd_->clear();  // graphs that keep the state point into the old state buffers
+        auto ed = ensure_decode(batch, &moved);  // allocate outside any capture
+        if (moved && fwd_) fwd_->clear();  // graphs that keep the state point into the old state buffers
+        if (!ed.ok()) return ed.error();
         dec_->steps = 0;
     }
     if (!fwd_) fwd_ = new FwdGraphs();
@@ -838,7 +941,7 @@ Result<Unit> ByteLM::run_layers(const uint8_t *tokens_dev, void *logits_dev, int
     for (auto &c : fwd_->entries)
         if (c.tok == tokens_dev && c.logits == logits_dev && c.batch == batch && c.seq_len == seq_len && c.keep == keep_state) e = &c;
     if (!e) {
-        if (fwd_->entries.size() >= 4) {  // drop the least recently used
+        if (fwd_->entries.size() >= kForwardGraphs) {  // drop the least recently used
             size_t lru = 0;
             for (size_t i = 1; i < fwd_->entries.size(); ++i)
                 if (fwd_->entries[i].used < fwd_->entries[lru].used) lru = i;
@@ -885,9 +988,9 @@ Result<Unit> ByteLM::run_layers(const uint8_t *tokens_dev, void *logits_dev, int
 
 Result<Unit> ByteLM::run_layers_plain(const uint8_t *tokens_dev, void *logits_dev, int64_t batch, int64_t seq_len, void *stream,
                                       bool keep_state) {
-    HELIX_TRY(ensure_buffers(batch, seq_len));
+    HELIX_TRY(ensure_buffers(batch, seq_len, nullptr));
     if (keep_state) {
-        HELIX_TRY(ensure_decode(batch));
+        HELIX_TRY(ensure_decode(batch, nullptr));
         dec_->steps = 0;
     }
     const int64_t T = batch * seq_len;
@@ -943,7 +1046,11 @@ Result<Unit> ByteLM::forward_host(const uint8_t *tokens_host, void *logits_host,
     std::lock_guard<std::recursive_mutex> lock(mu_);
     if (!tokens_host || !logits_host) return err(HX_ERR_INVALID_INPUT, "ByteLM::forward_host: NULL buffer");
     HELIX_TRY(use_device(device_));
-    HELIX_TRY(ensure_buffers(batch, seq_len));
+    if (batch <= 0 || seq_len <= 0) return err(HX_ERR_INVALID_DIMENSION, "ByteLM: batch and seq_len must be positive");
+    bool moved = false;
+    auto eb = ensure_buffers(batch, seq_len, &moved);
+    if (moved && fwd_) fwd_->clear();
+    if (!eb.ok()) return eb.error();
     const int64_t T = batch * seq_len;
     HELIX_TRY_ABI(hx_memcpy_h2d(buf_->tokens.data(), tokens_host, (size_t)T, stream));
     HELIX_TRY(forward_device(static_cast<const uint8_t *>(buf_->tokens.data()), buf_->logits.data(), batch, seq_len, stream));
@@ -957,7 +1064,7 @@ Result<DeviceTensor> ByteLM::forward(const DeviceTensor &tokens) const {
     if (tokens.ndim() != 2) return err(HX_ERR_SHAPE_MISMATCH, "ByteLM: expected tokens [batch, seq_len], got " + shape_str(tokens.shape()));
     const int64_t B = tokens.shape().dim(0), L = tokens.shape().dim(1);
     DeviceTensor logits;
-    HELIX_ASSIGN(logits, DeviceTensor::empty(Shape({B, L, 256}), dtype, device_));
+    HELIX_ASSIGN(logits, DeviceTensor::pooled(Shape({B, L, 256}), dtype, device_));
     if (B * L == 0) return logits;
     // forward() is const in the interface; the activation buffers are a cache
     HELIX_TRY(const_cast<ByteLM *>(this)->forward_device(static_cast<const uint8_t *>(tokens.data()), logits.data(), B, L, nullptr));
@@ -1007,7 +1114,7 @@ hx_status hx_tensor_from_host(const float *data, const int64_t *dims, int32_t nd
     HX_REQUIRE(out && (dims || ndim == 0) && ndim >= 0 && ndim <= 8, HX_ERR_INVALID_INPUT, "hx_tensor_from_host: bad arguments");
     HX_REQUIRE(dtype == HX_F32 || dtype == HX_BF16, HX_ERR_DTYPE_MISMATCH, "hx_tensor_from_host: dtype must be F32 or BF16");
     helix::Shape shape(std::vector<int64_t>(dims, dims + ndim));
-    auto r = helix::DeviceTensor::from_host_f32(data, shape, (helix::DType)dtype, dev_of(device_id));
+    auto r = helix::DeviceTensor::from_host_f32(data, shape, (helix::DType)dtype, dev_of(device_id), true);
     HX_RETURN_IF_ERR(r);
     *out = new hx_tensor{std::move(r.value())};
     return HX_OK;
@@ -1046,7 +1153,7 @@ hx_status hx_tensor_info(const hx_tensor *t, int32_t *ndim, int64_t *dims8, int3
     return HX_OK;
 }
 
-void *hx_tensor_data(const hx_tensor *t) { return t ? t->t.data() : nullptr; }
+void *hx_tensor_data(const hx_tensor *t) { return t ? t->t.data_for_caller() : nullptr; }
 
 void hx_tensor_free(hx_tensor *t) { delete t; }
 

@@ -89,9 +89,16 @@ class DeviceTensor {
   public:
     DeviceTensor() = default;
     static Result<DeviceTensor> empty(const Shape &shape, DType dtype, const Device &device);
+    // The same from the block cache (hx::pool_alloc): for tensors a call makes and drops and that only the module
+    // layer's own kernels touch, all of them queued on the legacy default stream.
+    static Result<DeviceTensor> pooled(const Shape &shape, DType dtype, const Device &device);
     static Result<DeviceTensor> zeros(const Shape &shape, DType dtype, const Device &device);
+    // The address for code outside this library, which may use it on any stream: the work queued so far is complete
+    // when this returns, and the block goes back with cudaFree, which waits for every stream, instead of to the cache.
+    void *data_for_caller() const;
     // host data is fp32 (or bytes for U8); it is converted to `dtype` on the way in
-    static Result<DeviceTensor> from_host_f32(const float *data, const Shape &shape, DType dtype, const Device &device);
+    static Result<DeviceTensor> from_host_f32(const float *data, const Shape &shape, DType dtype, const Device &device,
+                                              bool from_pool = false);
     static Result<DeviceTensor> from_host_u8(const uint8_t *data, const Shape &shape, const Device &device);
     Result<Unit> copy_from_host_f32(const float *data, int64_t n);
     Result<Unit> to_host_f32(float *out, int64_t n) const;  // widens bf16
@@ -107,7 +114,9 @@ class DeviceTensor {
     bool defined() const { return storage_ != nullptr || shape_.numel() == 0; }
 
   private:
-    std::shared_ptr<void> storage_;
+    struct Storage;
+    bool may_return_early(const void *host) const;
+    std::shared_ptr<Storage> storage_;
     void *ptr_ = nullptr;
     Shape shape_;
     DType dtype_ = DType::F32;
@@ -288,8 +297,8 @@ class ByteLM : public Module {
     float eps = 1e-5f;
 
   private:
-    Result<Unit> ensure_buffers(int64_t batch, int64_t seq_len);
-    Result<Unit> ensure_decode(int64_t batch);
+    Result<Unit> ensure_buffers(int64_t batch, int64_t seq_len, bool *moved);
+    Result<Unit> ensure_decode(int64_t batch, bool *moved);
     Result<Unit> enqueue_step(void *stream);
     Result<Unit> run_layers(const uint8_t *tokens_dev, void *logits_dev, int64_t batch, int64_t seq_len, void *stream,
                             bool keep_state);
@@ -318,9 +327,11 @@ class ByteLM : public Module {
 void manual_seed(uint64_t seed);
 
 // TensorRandom::{random_normal, random_uniform, random_bernoulli} (crates/tensor-core/src/tensor.rs:212-221)
-Result<DeviceTensor> init_normal(const Shape &shape, double stddev, DType dtype, const Device &device, double mean = 0.0);
-Result<DeviceTensor> init_uniform(const Shape &shape, double lo, double hi, DType dtype, const Device &device);
-Result<DeviceTensor> init_bernoulli(const Shape &shape, double p, DType dtype, const Device &device);
+Result<DeviceTensor> init_normal(const Shape &shape, double stddev, DType dtype, const Device &device, double mean = 0.0,
+                                 bool from_pool = false);
+Result<DeviceTensor> init_uniform(const Shape &shape, double lo, double hi, DType dtype, const Device &device,
+                                  bool from_pool = false);
+Result<DeviceTensor> init_bernoulli(const Shape &shape, double p, DType dtype, const Device &device, bool from_pool = false);
 
 // The tensor primitives the reference's generic blocks call on T (csrc/tensor_ops.cu): TensorOps
 // (tensor.rs:62-134), TensorBroadcast (:137-149), TensorActivation (:191-209), TensorMixedPrecision::cast (:238),

@@ -1,6 +1,8 @@
 // Library-level entry points: version, error strings, device memory and copies.
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <unordered_map>
 
 #include "hx_common.cuh"
 
@@ -28,6 +30,100 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+// ---- block cache of the module layer's tensors: whole cudaMalloc blocks, one free list per device keyed by size
+namespace {
+struct Pool {
+    std::mutex mu;
+    std::multimap<size_t, void *> free_blocks;         // size -> block
+    std::unordered_map<void *, size_t> size_of;        // every block of this device, cached or in use
+    size_t cached = 0;
+};
+Pool *pool_of(int dev) {
+    static Pool pools[64];
+    return dev >= 0 && dev < 64 ? &pools[dev] : nullptr;
+}
+// small sizes in steps of 512 bytes, large ones in steps of 1/8 of their power of two: the shapes of one workload
+// differ by a few rows and should land in the same block
+size_t pool_round(size_t bytes) {
+    size_t step = 512;
+    while (step * 16 < bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+}
+struct OnDevice {  // makes `dev` current for a scope
+    int prev = -1;
+    explicit OnDevice(int dev) {
+        int cur = 0;
+        if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) prev = cur;
+    }
+    ~OnDevice() {
+        if (prev >= 0) cudaSetDevice(prev);
+    }
+};
+}  // namespace
+
+void pool_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    Pool *p = pool_of(dev);
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(p->mu);
+    for (auto &b : p->free_blocks) {
+        p->size_of.erase(b.second);
+        cudaFree(b.second);
+    }
+    p->free_blocks.clear();
+    p->cached = 0;
+}
+
+hx_status pool_alloc(void **dptr, size_t bytes) {
+    *dptr = nullptr;
+    if (bytes == 0) return HX_OK;
+    int dev = 0;
+    HX_CUDA(cudaGetDevice(&dev));
+    Pool *p = pool_of(dev);
+    if (!p) return hx_alloc(dptr, bytes);
+    const size_t want = pool_round(bytes);
+    {
+        std::lock_guard<std::mutex> lock(p->mu);
+        auto it = p->free_blocks.lower_bound(want);
+        if (it != p->free_blocks.end() && it->first <= want + want / 4) {  // close enough in size
+            *dptr = it->second;
+            p->cached -= it->first;
+            p->free_blocks.erase(it);
+            return HX_OK;
+        }
+    }
+    hx_status s = hx_alloc(dptr, want);
+    if (s != HX_OK) return s;
+    std::lock_guard<std::mutex> lock(p->mu);
+    p->size_of[*dptr] = want;
+    return HX_OK;
+}
+
+void pool_discard(void *dptr, int device) {
+    if (!dptr) return;
+    if (Pool *p = pool_of(device)) {
+        std::lock_guard<std::mutex> lock(p->mu);
+        p->size_of.erase(dptr);
+    }
+    OnDevice scope(device);
+    cudaFree(dptr);
+}
+
+void pool_release(void *dptr, int device) {
+    if (!dptr) return;
+    if (Pool *p = pool_of(device)) {
+        std::lock_guard<std::mutex> lock(p->mu);
+        auto it = p->size_of.find(dptr);
+        if (it != p->size_of.end() && p->cached + it->second <= kPoolCachedBytes) {
+            p->free_blocks.emplace(it->second, dptr);
+            p->cached += it->second;
+            return;
+        }
+    }
+    pool_discard(dptr, device);
 }
 
 }  // namespace hx
@@ -75,6 +171,11 @@ hx_status hx_alloc(void **dptr, size_t bytes) {
     *dptr = nullptr;
     if (bytes == 0) return HX_OK;
     cudaError_t e = cudaMalloc(dptr, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // the memory may be in the module layer's block cache
+        cudaGetLastError();
+        hx::pool_trim();
+        e = cudaMalloc(dptr, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return hx::fail(HX_ERR_ALLOCATION_FAILED, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));

@@ -42,6 +42,18 @@ inline size_t dtype_size(int dt) { return dt == HX_F32 ? 4 : dt == HX_BF16 ? 2 :
 // Number of SMs of the current device, cached per device.
 int sm_count();
 
+// Device memory for the tensors the module layer makes and drops on every call (results, workspaces, uploaded inputs).
+// cudaMalloc and cudaFree cost 0.1 to several ms each and cudaFree waits for the whole device; a freed block is kept
+// here instead and handed to the next request of about its size.  Both calls may come from any thread.  A block may
+// only be returned when everything that touches it was queued on the legacy default stream (stream order is what
+// keeps the next owner's work behind it).  At most kPoolCachedBytes per device stay cached; what goes beyond that and
+// everything on an allocation failure is given back with cudaFree.
+constexpr size_t kPoolCachedBytes = (size_t)512 << 20;
+hx_status pool_alloc(void **dptr, size_t bytes);
+void pool_release(void *dptr, int device);   // back to the cache; `device` is where it was allocated
+void pool_discard(void *dptr, int device);   // a real cudaFree (waits for the device)
+void pool_trim();                            // gives every cached block of the current device back
+
 // resid[i] += x[i] (x fp32 or bf16): the residual update where no GEMM epilogue can do it.
 hx_status residual_add(float *resid, const void *x, int x_dtype, int64_t n, cudaStream_t st);
 

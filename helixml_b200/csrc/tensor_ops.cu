@@ -140,7 +140,7 @@ template <typename T> __global__ void gather_kernel(const T *a, T *o, int64_t n,
 }
 
 Result<DeviceTensor> gather(const DeviceTensor &a, const Shape &out_shape, const Gather &g) {
-    auto out = DeviceTensor::empty(out_shape, a.dtype(), a.device());
+    auto out = DeviceTensor::pooled(out_shape, a.dtype(), a.device());
     if (!out.ok()) return out.error();
     const int64_t n = out_shape.numel();
     if (n == 0) return out;
@@ -191,7 +191,7 @@ Result<DeviceTensor> binary(int op, const DeviceTensor &a, const DeviceTensor &b
     if (a.dtype() != b.dtype() || !is_float(a.dtype())) return terr(HX_ERR_DTYPE_MISMATCH, "binary op needs two F32 or two BF16 tensors");
     if (!(a.device() == b.device())) return terr(HX_ERR_DEVICE_MISMATCH, "binary op on tensors of different devices");
     TOPS_TRY(on_device(a));
-    auto out = DeviceTensor::empty(a.shape(), a.dtype(), a.device());
+    auto out = DeviceTensor::pooled(a.shape(), a.dtype(), a.device());
     if (!out.ok()) return out.error();
     const int64_t n = a.numel();
     if (n == 0) return out;
@@ -210,7 +210,7 @@ Result<DeviceTensor> unary(int op, const DeviceTensor &a, float p0, float p1) {
     if (op < HX_OP_SQRT || op > HX_OP_LEAKY_RELU) return terr(HX_ERR_INVALID_INPUT, "unknown unary op " + std::to_string(op));
     if (!is_float(a.dtype())) return terr(HX_ERR_DTYPE_MISMATCH, "unary op needs an F32 or BF16 tensor");
     TOPS_TRY(on_device(a));
-    auto out = DeviceTensor::empty(a.shape(), a.dtype(), a.device());
+    auto out = DeviceTensor::pooled(a.shape(), a.dtype(), a.device());
     if (!out.ok()) return out.error();
     const int64_t n = a.numel();
     if (n == 0) return out;
@@ -244,7 +244,7 @@ Result<DeviceTensor> matmul(const DeviceTensor &a, const DeviceTensor &b) {
     if (K != Kb) return terr(HX_ERR_SHAPE_MISMATCH, "matmul inner dimensions " + std::to_string(K) + " and " + std::to_string(Kb));
     if (M > 0x7fffffff || N > 0x7fffffff || K > 0x7fffffff) return terr(HX_ERR_INVALID_DIMENSION, "matmul dimension exceeds 2^31");
     TOPS_TRY(on_device(a));
-    auto out = DeviceTensor::empty(out_shape, a.dtype(), a.device());
+    auto out = DeviceTensor::pooled(out_shape, a.dtype(), a.device());
     if (!out.ok()) return out.error();
     if (M * N == 0) return out;
     if (hx_matmul_ref(a.data(), b.data(), out.value().data(), (int)M, (int)N, (int)K, (int)a.dtype(), nullptr) != HX_OK)
@@ -292,7 +292,7 @@ Result<DeviceTensor> slice(const DeviceTensor &a, const std::vector<int64_t> &st
 static Result<DeviceTensor> concat_buffers(const std::vector<const DeviceTensor *> &ts, const Shape &out_shape) {
     const DeviceTensor &f = *ts[0];
     TOPS_TRY(on_device(f));
-    auto out = DeviceTensor::empty(out_shape, f.dtype(), f.device());
+    auto out = DeviceTensor::pooled(out_shape, f.dtype(), f.device());
     if (!out.ok()) return out.error();
     size_t off = 0;
     const size_t es = dtype_size(f.dtype());
@@ -382,7 +382,7 @@ Result<DeviceTensor> cast(const DeviceTensor &a, DType dtype) {
     if (!is_float(a.dtype()) || !is_float(dtype)) return terr(HX_ERR_UNSUPPORTED_OPERATION, "cast between F32 and BF16 only");
     if (a.dtype() == dtype) return a.clone();
     TOPS_TRY(on_device(a));
-    auto out = DeviceTensor::empty(a.shape(), dtype, a.device());
+    auto out = DeviceTensor::pooled(a.shape(), dtype, a.device());
     if (!out.ok()) return out.error();
     const int64_t n = a.numel();
     if (n == 0) return out;
@@ -404,7 +404,7 @@ Result<float> to_scalar(const DeviceTensor &a) {
 
 Result<DeviceTensor> full(float value, const Shape &shape, DType dtype, const Device &device) {
     if (!is_float(dtype)) return terr(HX_ERR_DTYPE_MISMATCH, "full: dtype must be F32 or BF16");
-    auto out = DeviceTensor::empty(shape, dtype, device);
+    auto out = DeviceTensor::pooled(shape, dtype, device);
     if (!out.ok()) return out.error();
     const int64_t n = shape.numel();
     if (n == 0) return out;
@@ -418,7 +418,7 @@ Result<DeviceTensor> eye(int64_t n, DType dtype, const Device &device) {
     if (n < 0) return terr(HX_ERR_INVALID_DIMENSION, "eye: negative size");
     std::vector<float> h((size_t)n * n, 0.f);
     for (int64_t i = 0; i < n; ++i) h[(size_t)i * n + i] = 1.f;
-    return DeviceTensor::from_host_f32(h.data(), Shape({n, n}), dtype, device);
+    return DeviceTensor::from_host_f32(h.data(), Shape({n, n}), dtype, device, true);
 }
 
 Result<DeviceTensor> arange(float start, float end, float step, DType dtype, const Device &device) {
@@ -429,7 +429,7 @@ Result<DeviceTensor> arange(float start, float end, float step, DType dtype, con
         if (h.size() > (size_t)1 << 28) return terr(HX_ERR_INVALID_INPUT, "arange of more than 2^28 elements");
         h.push_back(cur);
     }
-    return DeviceTensor::from_host_f32(h.data(), Shape({(int64_t)h.size()}), dtype, device);
+    return DeviceTensor::from_host_f32(h.data(), Shape({(int64_t)h.size()}), dtype, device, true);
 }
 
 }  // namespace tops
@@ -568,11 +568,11 @@ hx_status hx_tensor_random(int32_t kind, const int64_t *dims, int32_t ndim, floa
     HX_REQUIRE(out && shape_from(dims, ndim, &s), HX_ERR_INVALID_INPUT, "hx_tensor_random: bad arguments");
     const helix::Device dev = helix::Device::cuda(device_id);
     switch (kind) {
-        case HX_RANDOM_NORMAL: return give(helix::init_normal(s, (double)p1, helix::DType::F32, dev, (double)p0), out);
+        case HX_RANDOM_NORMAL: return give(helix::init_normal(s, (double)p1, helix::DType::F32, dev, (double)p0, true), out);
         case HX_RANDOM_UNIFORM:
             HX_REQUIRE(p0 < p1, HX_ERR_INVALID_INPUT, "hx_tensor_random: empty range [%g, %g)", p0, p1);
-            return give(helix::init_uniform(s, (double)p0, (double)p1, helix::DType::F32, dev), out);
-        case HX_RANDOM_BERNOULLI: return give(helix::init_bernoulli(s, (double)p0, helix::DType::F32, dev), out);
+            return give(helix::init_uniform(s, (double)p0, (double)p1, helix::DType::F32, dev, true), out);
+        case HX_RANDOM_BERNOULLI: return give(helix::init_bernoulli(s, (double)p0, helix::DType::F32, dev, true), out);
         default: return hx::fail(HX_ERR_INVALID_INPUT, "hx_tensor_random: unknown kind %d", kind);
     }
 }

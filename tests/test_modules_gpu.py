@@ -451,3 +451,50 @@ def test_sequential_chains_modules():
     assert e.value.variant == "ShapeMismatch"
     empty = nn.Sequential()
     assert len(empty) == 0 and np.array_equal(empty(nn.Tensor.from_numpy(x)).numpy(), x)
+
+
+@pytest.mark.parametrize("lengths", [(64, 200, 33), (300, 7, 300, 120)])
+def test_byte_lm_changing_lengths_share_buffers(lengths):
+    """Prompts of changing length (shrinking, growing past the buffers, repeated) and batch give what a model that
+    never saw another shape gives, captured or not, and a decode step follows each prefill."""
+    import torch
+    from helixml_b200 import nn
+    emb, layers, normf = _lm_weights(17, 2, 128)
+
+    def fresh():
+        lm = nn.ByteLM(2, 128)
+        lm.load_weights(emb, layers, normf)
+        return lm
+
+    def run(lm, B, L, i):
+        tok = torch.from_numpy(synth.random_bytes(17, f"t{i}", (B, L))).cuda()
+        nxt = torch.from_numpy(synth.random_bytes(17, f"n{i}", (B,))).cuda()
+        out = torch.empty(B, L, 256, device="cuda", dtype=torch.bfloat16)
+        lg = torch.empty(B, 256, device="cuda", dtype=torch.bfloat16)
+        lm.prefill_device(tok.data_ptr(), out.data_ptr(), B, L)
+        lm.decode_step_device(nxt.data_ptr(), lg.data_ptr(), B)
+        torch.cuda.synchronize()
+        return out, lg
+
+    shapes = [(1 + i % 3, L) for i, L in enumerate(lengths)]
+    want = [run(fresh(), B, L, i) for i, (B, L) in enumerate(shapes)]
+    lm = fresh()
+    for rnd in range(3):
+        for i, (B, L) in enumerate(shapes):
+            got = run(lm, B, L, i)
+            assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), (rnd, i)
+
+
+def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
+    """A result's memory returns to the block cache and the next result of its size is correct; an address handed to the
+    caller keeps its contents while other results come and go."""
+    import torch
+    from helixml_b200 import nn
+    a = np.arange(12345, dtype=np.float32)
+    kept = nn.Tensor.from_numpy(a).add_scalar(1.0)
+    assert kept.data_ptr() != 0
+    for i in range(20):
+        t = nn.Tensor.from_numpy(a * i)
+        assert np.array_equal(t.mul_scalar(2.0).numpy(), a * i * 2)
+    torch.cuda.synchronize()
+    assert np.array_equal(kept.numpy(), a + 1)
