@@ -54,10 +54,12 @@ static Layout plan(const hx_mamba_block_args *a) {
     l.y = off; off += up(T * E * es);
     // carries of a split scan (the split evens out the load; see hx_selective_scan_suggest_splits)
     hx_scan_args sa = scan_shape(a);
-    // variants that chain their segments are planned as such (the parallel-segment suggestion is for the look-back form)
+    // variants that chain their segments are planned as such (the parallel-segment suggestion is for the look-back form,
+    // which does not take a ready-made gate)
     if (a->scan_variant == HX_SCAN_TILED || a->scan_variant == HX_SCAN_SEQSPLIT || a->scan_variant == HX_SCAN_DIRECT)
-        sa.a_geometric = 0;
+        sa.z_is_gate = 1;
     l.splits = (a->scan_variant == HX_SCAN_SIMPLE || a->d_state != 16) ? 1 : hx_selective_scan_suggest_splits(&sa);
+    sa.z_is_gate = 0;
     sa.seq_splits = l.splits;
     l.scan_ws_bytes = 0;
     if (l.splits > 1) hx_selective_scan_workspace_bytes(&sa, &l.scan_ws_bytes);
@@ -98,7 +100,7 @@ static bool fuses_dt(const hx_mamba_block_args *a, int W, int splits) {
     // a dt_proj kernel of its own.
     const hx::scan::ScanKind kind = hx::scan::auto_kind(&sa);
     if (kind == hx::scan::ScanKind::Direct) return HX_BLOCK_FUSE_DT_AUTO >= 1 && hx::scan::auto_channels_per_lane(&sa) == 1;
-    if (kind == hx::scan::ScanKind::LookBack) return HX_BLOCK_FUSE_DT_AUTO >= 2 && a->a_geometric != 0;
+    if (kind == hx::scan::ScanKind::LookBack) return HX_BLOCK_FUSE_DT_AUTO >= 2;
     return false;
 }
 

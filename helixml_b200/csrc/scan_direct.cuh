@@ -24,12 +24,13 @@
 //
 // Split sequences come in two forms.  MODE 0 chains the segments: segment s+1 starts from the state segment s
 // hands over (carry + flag), so the segments of one chain run one after the other; that evens out the load when
-// chains are plentiful.  MODES 1 and 2 are the look-back form for few chains (geometric A only), two launches in
-// stream order with no flag between CTAs:
+// chains are plentiful.  MODES 1 and 2 are the look-back form for few chains, two launches in stream order with no flag
+// between CTAs:
 //   MODE 1, the aggregate pass, runs segments 0 .. S-2 at the same time, each from a zero state and backwards in
 //           time: with w_t = exp2(A0 * sum_{tau > t} dt_tau) the end state is q[n] = sum_t (dt_t u_t w_t^(n+1)) B_t[n],
 //           i.e. one multiply for the power (the input is folded into the chain of powers) and one FMA per state,
-//           no C contraction, no gate, no output.  It writes q and sum(dt) per (segment, chain).
+//           no C contraction, no gate, no output.  It writes q and sum(dt) per (segment, chain).  For a general A, where
+//           each state has an exponential of its own, it runs the forward recurrence without outputs instead.
 //   MODE 2, the output pass, runs all S segments at the same time: a segment first folds the aggregates of its
 //           predecessors, h <- exp(A sum dt_j) h + q_j for j = 0 .. s-1 (the look-back), then scans its steps
 //           with outputs like MODE 0.
@@ -55,6 +56,9 @@
 #ifndef HX_SCAN_FULL_UNROLL
 #define HX_SCAN_FULL_UNROLL 1
 #endif
+#ifndef HX_SCAN_MINB_GENERAL
+#define HX_SCAN_MINB_GENERAL 4
+#endif
 #ifndef HX_SCAN_MINB_LOOKBACK
 #define HX_SCAN_MINB_LOOKBACK 0
 #endif
@@ -62,9 +66,13 @@
 namespace hx {
 namespace scan {
 
-template <typename T, int CPL_, bool GEOM_, bool STD_, int STAGES_, int FUSEDT_ = 0, bool ZGATE_ = false,
+// GEOM_: 1 = A[d][n] is (n + 1) A[d][0] (the caller's assertion), 0 = general A, 2 = each CTA looks at the A rows of its
+// own channels and takes the form they allow.
+template <typename T, int CPL_, int GEOM_, bool STD_, int STAGES_, int FUSEDT_ = 0, bool ZGATE_ = false,
           bool BLOCK_ = false, int MODE_ = 0>
 struct DirectCfg {
+    template <int G> using WithGeom = DirectCfg<T, CPL_, G, STD_, STAGES_, FUSEDT_, ZGATE_, BLOCK_, MODE_>;
+    static constexpr int GEOM_FORM = GEOM_;
     static constexpr int MODE = MODE_;                 // 0 chained segments, 1 aggregate pass, 2 output pass (see above)
     static constexpr bool BLOCK = BLOCK_;              // the Mamba block's call: no conv (u is given), gate and softplus
                                                        // present, all known at compile time
@@ -78,7 +86,7 @@ struct DirectCfg {
     static constexpr int TMEM_COLS = STAGES_ * 16 <= 32 ? 32 : 64;   // FUSEDT == 2: STAGES accumulators of TC columns
     static constexpr int RP = 64;                      // columns of the dt_low / W_dt tiles (dt_rank <= 64, zero filled)
     static constexpr int CPL = CPL_;
-    static constexpr bool GEOM = GEOM_;
+    static constexpr bool GEOM = GEOM_ == 1;
     static constexpr bool STD = STD_;
     static constexpr bool FAST = sizeof(T) == 2;
     static constexpr int ES = sizeof(T);
@@ -95,7 +103,9 @@ struct DirectCfg {
     static constexpr int UNROLL = HX_SCAN_UNROLL;
     static constexpr bool FULL = FUSEDT_ == 2 || (HX_SCAN_FULL_UNROLL && CPL_ == 1);   // whole chunks fully unrolled
     static constexpr int REM_UNROLL = FULL ? 1 : HX_SCAN_UNROLL;                       // the loop they do not take
-    static constexpr int MIN_CTAS = (MODE_ != 0 && !FUSEDT_) ? HX_SCAN_MINB_LOOKBACK : HX_SCAN_MINB_CHAINED;
+    // with a general A the unrolled chunk would take 250 registers (the exponentials of many steps in flight), one CTA per SM
+    static constexpr int MIN_CTAS = GEOM_ != 1 ? (CPL_ == 2 ? 2 : MODE_ != 0 ? HX_SCAN_MINB_GENERAL : 3)
+                                    : (MODE_ != 0 && !FUSEDT_) ? HX_SCAN_MINB_LOOKBACK : HX_SCAN_MINB_CHAINED;
     static constexpr int X_BYTES = (TC + 3) * 128;
     static constexpr int ROW_BYTES = TC * 128;
     static constexpr int DTROW = FUSEDT == 1 ? BOXC * 4 + 32 : 128;       // bytes per dt row (fp32 + pad when produced here:
@@ -114,7 +124,6 @@ struct DirectCfg {
     static_assert(!FUSEDT || sizeof(T) == 2, "the fused dt projection takes bf16 operands");
     static_assert(FUSEDT != 2 || (CPL_ == 1 && DT == 128 && STAGES_ * TC <= TMEM_COLS),
                   "the tensor-memory form maps channel c of the CTA to accumulator lane c");
-    static_assert(MODE == 0 || GEOM, "the look-back passes need geometric A");
 };
 
 template <typename T> __device__ __forceinline__ float2 ld_chan2(const char *p);  // two adjacent channels
@@ -129,13 +138,28 @@ template <> __device__ __forceinline__ float ld_chan1<__nv_bfloat16>(const char 
     return __uint_as_float((uint32_t)(*reinterpret_cast<const uint16_t *>(p)) << 16);
 }
 
+// The rule of hx_scan_check_geometric on the A rows of the CTA's channels (every thread of the CTA calls this).
+template <typename Cfg> __device__ __forceinline__ bool cta_is_geometric(const TiledParams &p) {
+    const int n = min(Cfg::DT, p.D - (int)blockIdx.x * Cfg::DT);
+    bool ok = true;
+    for (int c = threadIdx.x; c < n; c += Cfg::THREADS) {
+        const float *row = p.A + ((int64_t)blockIdx.x * Cfg::DT + c) * 16;
+        const float a0 = row[0];
+        if (!(a0 <= 0.f)) ok = false;
+#pragma unroll
+        for (int i = 1; i < 16; ++i) {
+            const float want = (float)(i + 1) * a0;
+            if (fabsf(row[i] - want) > 1e-6f * fabsf(want)) ok = false;
+        }
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
 template <typename T, typename Cfg>
-__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS)
-scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dt,
-                   const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_B,
-                   const __grid_constant__ CUtensorMap tm_C, const __grid_constant__ CUtensorMap tm_dtlow,
-                   const __grid_constant__ CUtensorMap tm_wdt, const TiledParams p, T *__restrict__ yg, const int64_t y_bs,
-                   const int64_t y_rs) {
+__device__ __forceinline__ void
+scan_direct_body(const CUtensorMap &tm_x, const CUtensorMap &tm_dt, const CUtensorMap &tm_z, const CUtensorMap &tm_B,
+                 const CUtensorMap &tm_C, const CUtensorMap &tm_dtlow, const CUtensorMap &tm_wdt, const TiledParams &p,
+                 T *__restrict__ yg, const int64_t y_bs, const int64_t y_rs) {
     constexpr int CPL = Cfg::CPL, TC = Cfg::TC, STAGES = Cfg::STAGES, NW = Cfg::NWARP, NB = Cfg::NB, ES = Cfg::ES;
     constexpr bool GEOM = Cfg::GEOM, FAST = Cfg::FAST, STD = Cfg::STD;
     constexpr int FUSEDT = Cfg::FUSEDT;
@@ -223,7 +247,7 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
         auto issue = [&](int i) {
             const int s = i % STAGES;
-            const int t0 = t_seg0 + (MODE == 1 ? nchunks - 1 - i : i) * TC;  // the aggregate pass walks backwards
+            const int t0 = t_seg0 + (MODE == 1 && GEOM ? nchunks - 1 - i : i) * TC;  // the geometric aggregate pass walks backwards
             const uint32_t sb = smem_u32(stage_base + s * Cfg::STAGE_BYTES);
             mbar_expect_tx(bar_full(s), stage_tx);
             for (int bx = 0; bx < live_boxes; ++bx) {
@@ -396,7 +420,7 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 8; ++j) h[e][j] = make_float2(0.f, 0.f);
 
-    if constexpr (MODE == 1) {
+    if constexpr (MODE == 1 && GEOM) {
         // ============================================================ aggregate pass (look-back form)
         // End state of this segment from a zero state, walking backwards: w = exp2(A0 * (sum of dt after t)) is the
         // decay from step t to the end of the segment, and q[n] += (dt_t u_t w^(n+1)) B_t[n].
@@ -475,9 +499,7 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                         dtv = v;
                     }
                     const float xin = dtv * u;
-                    float r;
-                    if constexpr (FAST) r = ex2_approx(sacc[e] * a0_[e]);
-                    else r = exp2f(sacc[e] * a0_[e]);
+                    const float r = ex2_approx(sacc[e] * a0_[e]);
                     sacc[e] += dtv;
                     const float r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
                     float2 a[8];
@@ -527,6 +549,10 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         return;
     }
 
+    constexpr bool AGG = MODE == 1;  // from here on: the aggregate pass of a general A (no C, no gate, no output)
+    float sacc[CPL];                 // its sum of dt
+#pragma unroll
+    for (int e = 0; e < CPL; ++e) sacc[e] = 0.f;
     if constexpr (MODE == 2) {
         // ============================================================ look-back: fold the predecessors' aggregates
         if (seg > 0) {
@@ -537,21 +563,44 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 const float2 *q0 = reinterpret_cast<const float2 *>(p.carry + c0 * 16);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) h[e][j] = q0[j];  // segment 0 starts from zero: its aggregate is its end state
-                for (int js = 1; js < seg; ++js) {
-                    const float sd = p.sdt[c0 + js * cs];
-                    float r;
-                    if constexpr (FAST) r = ex2_approx(sd * a0_[e]);
-                    else r = exp2f(sd * a0_[e]);
-                    float2 a[8];
-                    a[0] = make_float2(r, r * r);
-                    a[1] = mul2(a[0], splat2(a[0].y));
-                    a[2] = mul2(a[0], splat2(a[1].y));
-                    a[3] = mul2(a[1], splat2(a[1].y));
+                // Four aggregates are fetched before the first is used: one at a time a segment with many predecessors
+                // waits out a trip to L2 for each of them (20 us of an 80 us call at 32 segments).
+                constexpr int FB = 4;
+                for (int js = 1; js < seg; js += FB) {
+                    float2 qv[FB][8];
+                    float sd[FB];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) a[4 + j] = mul2(a[j], splat2(a[3].y));
-                    const float2 *qj = reinterpret_cast<const float2 *>(p.carry + (c0 + js * cs) * 16);
+                    for (int f = 0; f < FB; ++f) {
+                        const int jj = min(js + f, seg - 1);
+                        sd[f] = p.sdt[c0 + jj * cs];
+                        const float4 *qj = reinterpret_cast<const float4 *>(p.carry + (c0 + jj * cs) * 16);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) h[e][j] = fma2(a[j], h[e][j], qj[j]);
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 v = qj[j];
+                            qv[f][2 * j] = make_float2(v.x, v.y);
+                            qv[f][2 * j + 1] = make_float2(v.z, v.w);
+                        }
+                    }
+#pragma unroll
+                    for (int f = 0; f < FB; ++f) {
+                        if (js + f >= seg) break;
+                        float2 a[8];
+                        if constexpr (GEOM) {
+                            const float r = ex2_approx(sd[f] * a0_[e]);
+                            a[0] = make_float2(r, r * r);
+                            a[1] = mul2(a[0], splat2(a[0].y));
+                            a[2] = mul2(a[0], splat2(a[1].y));
+                            a[3] = mul2(a[1], splat2(a[1].y));
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) a[4 + j] = mul2(a[j], splat2(a[3].y));
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                a[j] = make_float2(ex2_approx(sd[f] * a2l[GEOM ? 0 : e][2 * j]), ex2_approx(sd[f] * a2l[GEOM ? 0 : e][2 * j + 1]));
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) h[e][j] = fma2(a[j], h[e][j], qv[f][j]);
+                    }
                 }
             }
         }
@@ -641,7 +690,7 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 Bv[k] = sBf[t * 4 + k];
-                Cv[k] = sCf[t * 4 + k];
+                if constexpr (!AGG) Cv[k] = sCf[t * 4 + k];
             }
             float yout[CPL];
 #pragma unroll
@@ -671,14 +720,14 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 } else {
                     dtv = v;
                 }
-                const float g = has_z ? (z_gate ? zr[e] : silu_sel<FAST>(zr[e])) : 1.f;
+                float g = 1.f;
+                if constexpr (!AGG) g = has_z ? (z_gate ? zr[e] : silu_sel<FAST>(zr[e])) : 1.f;
                 const float xin = dtv * u;
+                if constexpr (AGG) sacc[e] += dtv;
                 // ---- decays
                 float2 a[8];
                 if constexpr (GEOM) {
-                    float r;
-                    if constexpr (FAST) r = ex2_approx(dtv * a0_[e]);
-                    else r = exp2f(dtv * a0_[e]);
+                    const float r = ex2_approx(dtv * a0_[e]);
                     const float r2 = r * r;
                     a[0] = make_float2(r, r2);
                     a[1] = mul2(a[0], splat2(r2));
@@ -690,12 +739,8 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                     for (int j = 0; j < 4; ++j) a[4 + j] = mul2(a[j], splat2(r8));
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if constexpr (FAST)
-                            a[j] = make_float2(ex2_approx(dtv * a2l[GEOM ? 0 : e][2 * j]), ex2_approx(dtv * a2l[GEOM ? 0 : e][2 * j + 1]));
-                        else
-                            a[j] = make_float2(exp2f(dtv * a2l[GEOM ? 0 : e][2 * j]), exp2f(dtv * a2l[GEOM ? 0 : e][2 * j + 1]));
-                    }
+                    for (int j = 0; j < 8; ++j)
+                        a[j] = make_float2(ex2_approx(dtv * a2l[GEOM ? 0 : e][2 * j]), ex2_approx(dtv * a2l[GEOM ? 0 : e][2 * j + 1]));
                 }
                 // ---- recurrence and output contraction, four independent accumulators
                 const float2 x2 = splat2(xin);
@@ -704,12 +749,16 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 for (int k = 0; k < 4; ++k) {
                     h[e][2 * k] = fma2(a[2 * k], h[e][2 * k], mul2(x2, make_float2(Bv[k].x, Bv[k].y)));
                     h[e][2 * k + 1] = fma2(a[2 * k + 1], h[e][2 * k + 1], mul2(x2, make_float2(Bv[k].z, Bv[k].w)));
-                    acc[0] = fma2(make_float2(Cv[k].x, Cv[k].y), h[e][2 * k], acc[0]);
-                    acc[1] = fma2(make_float2(Cv[k].z, Cv[k].w), h[e][2 * k + 1], acc[1]);
+                    if constexpr (!AGG) {
+                        acc[0] = fma2(make_float2(Cv[k].x, Cv[k].y), h[e][2 * k], acc[0]);
+                        acc[1] = fma2(make_float2(Cv[k].z, Cv[k].w), h[e][2 * k + 1], acc[1]);
+                    }
                 }
+                if constexpr (AGG) continue;
                 const float2 ys = add2(acc[0], acc[1]);
                 yout[e] = (ys.x + ys.y + ds_[e] * u) * g;
             }
+            if constexpr (AGG) return;
             // y goes straight from registers to HBM: the warp writes one contiguous run of 32*CPL channels
             T *yp = yrow + (int64_t)t * y_rs;
             if constexpr (CPL == 2) {
@@ -750,12 +799,17 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         if (lane == 0) mbar_arrive(bar_empty(s));
     }
 
-    const bool last_seg = seg == p.n_segments - 1;
+    const bool last_seg = seg == p.n_segments - 1;  // (never in the aggregate pass)
 #pragma unroll
     for (int e = 0; e < CPL; ++e) {
         if (dch + e >= p.D) continue;
         float2 *dst = nullptr;
-        if (last_seg && p.h_last) dst = reinterpret_cast<float2 *>(p.h_last + ((int64_t)b * p.D + dch + e) * 16);
+        if (MODE != 1 && last_seg && p.h_last) dst = reinterpret_cast<float2 *>(p.h_last + ((int64_t)b * p.D + dch + e) * 16);
+        if (MODE == 1) {
+            const int64_t ci = ((int64_t)seg * p.B + b) * p.D + dch + e;
+            dst = reinterpret_cast<float2 *>(p.carry + ci * 16);
+            p.sdt[ci] = sacc[e];
+        }
         if (MODE == 0 && !last_seg) dst = reinterpret_cast<float2 *>(p.carry + (((int64_t)seg * p.B + b) * p.D + dch + e) * 16);
         if (dst) {
 #pragma unroll
@@ -772,6 +826,23 @@ scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     }
     if constexpr (FUSEDT == 2) {
         if (lane == 0) mbar_arrive(bar_tdone);
+    }
+}
+
+template <typename T, typename Cfg>
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS)
+scan_direct_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dt,
+                   const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_B,
+                   const __grid_constant__ CUtensorMap tm_C, const __grid_constant__ CUtensorMap tm_dtlow,
+                   const __grid_constant__ CUtensorMap tm_wdt, const __grid_constant__ TiledParams p, T *__restrict__ yg,
+                   const int64_t y_bs, const int64_t y_rs) {
+    if constexpr (Cfg::GEOM_FORM == 2) {
+        if (cta_is_geometric<Cfg>(p))
+            scan_direct_body<T, typename Cfg::template WithGeom<1>>(tm_x, tm_dt, tm_z, tm_B, tm_C, tm_dtlow, tm_wdt, p, yg, y_bs, y_rs);
+        else
+            scan_direct_body<T, typename Cfg::template WithGeom<0>>(tm_x, tm_dt, tm_z, tm_B, tm_C, tm_dtlow, tm_wdt, p, yg, y_bs, y_rs);
+    } else {
+        scan_direct_body<T, Cfg>(tm_x, tm_dt, tm_z, tm_B, tm_C, tm_dtlow, tm_wdt, p, yg, y_bs, y_rs);
     }
 }
 

@@ -760,7 +760,7 @@ static void seg_plan(const hx_scan_args *a, int chunk, int *n_seg, int *seg_len)
 }
 
 constexpr int kChunkBf16 = 32, kChunkF32 = 32;
-constexpr int kPlanChunk = 32;  // segment lengths are multiples of this
+constexpr int kPlanChunk = 32;  // segment lengths are multiples of this (of the direct kernel's 16 steps in the look-back form)
 
 static int tiles_of(const hx_scan_args *a) {
     const int DT = a->io_dtype == HX_BF16 ? 64 : 32;
@@ -823,7 +823,7 @@ static hx_status launch_tiled(const hx_scan_args *a, bool split, cudaStream_t st
     // `reserved` picks another (chunk, stages) pair for the bf16 / geometric / standard path (tuning knob)
     const bool stdp0 = a->conv_w != nullptr && a->z != nullptr && a->dt_softplus != 0;
     // only 1 and 2 name a tuning variant; anything else (the direct kernel's selector among them) is the default
-    const int tune = (bf && a->a_geometric && stdp0 && (a->reserved == 1 || a->reserved == 2)) ? a->reserved : 0;
+    const int tune = (bf && a->a_geometric == 1 && stdp0 && (a->reserved == 1 || a->reserved == 2)) ? a->reserved : 0;
     const int ES = bf ? 2 : 4, DT = 128 / ES, TC = tune >= 1 ? 16 : (bf ? kChunkBf16 : kChunkF32);
     const int tiles = (a->d_inner + DT - 1) / DT;
     int n_seg = 1, seg_len = (a->seq_len + TC - 1) / TC * TC;
@@ -885,7 +885,7 @@ static hx_status launch_tiled(const hx_scan_args *a, bool split, cudaStream_t st
                a->batch, n_seg);
     dim3 grid(tiles, a->batch, n_seg);
     const int lpc = choose_lpc(a);
-    const bool geom = a->a_geometric != 0;
+    const bool geom = a->a_geometric == 1;  // (2, decided on the device, is the one-lane-per-channel kernel's)
     // the standard path (4-tap conv, softplus, gate) has its flags fixed at compile time
     const bool stdp = a->conv_w != nullptr && a->z != nullptr && a->dt_softplus != 0;
 #define HX_TILED_CASE(T, LPC, GEOM, TCv, ST)                                                    \
@@ -929,7 +929,7 @@ static hx_status launch_tiled(const hx_scan_args *a, bool split, cudaStream_t st
 }
 
 
-template <typename T, int CPL, bool GEOM, bool STD, int STAGES = 2, int FUSEDT = 0, bool ZGATE = false, bool BLOCK = false,
+template <typename T, int CPL, int GEOM, bool STD, int STAGES = 2, int FUSEDT = 0, bool ZGATE = false, bool BLOCK = false,
           int MODE = 0>
 static hx_status launch_direct_inst(const TiledParams &p, const CUtensorMap *maps, dim3 grid, cudaStream_t st, void *y,
                                     int64_t y_bs, int64_t y_rs) {
@@ -949,26 +949,28 @@ static hx_status launch_direct_inst(const TiledParams &p, const CUtensorMap *map
 
 // The two launches of the look-back form: the aggregate pass over segments 0 .. S-2, then the output pass over
 // all S segments (stream order is the only dependency between them).
-template <typename T, bool STD, int FUSEDT, bool BLOCK>
-static hx_status launch_lookback_pair(const TiledParams &p, const CUtensorMap *maps, dim3 grid, cudaStream_t st, void *y,
+template <typename T, int GEOM, bool STD, int FUSEDT, bool BLOCK>
+static hx_status launch_lookback_geom(const TiledParams &p, const CUtensorMap *maps, dim3 grid, cudaStream_t st, void *y,
                                       int64_t y_bs, int64_t y_rs) {
     dim3 g1(grid.x, grid.y, grid.z - 1);
-    hx_status s = launch_direct_inst<T, 1, true, STD, 2, FUSEDT, false, BLOCK, 1>(p, maps, g1, st, y, y_bs, y_rs);
+    hx_status s = launch_direct_inst<T, 1, GEOM, STD, 2, FUSEDT, false, BLOCK, 1>(p, maps, g1, st, y, y_bs, y_rs);
     if (s != HX_OK) return s;
-    return launch_direct_inst<T, 1, true, STD, 2, FUSEDT, false, BLOCK, 2>(p, maps, grid, st, y, y_bs, y_rs);
+    return launch_direct_inst<T, 1, GEOM, STD, 2, FUSEDT, false, BLOCK, 2>(p, maps, grid, st, y, y_bs, y_rs);
+}
+template <typename T, bool STD, int FUSEDT, bool BLOCK>
+static hx_status launch_lookback_pair(int geom, const TiledParams &p, const CUtensorMap *maps, dim3 grid, cudaStream_t st, void *y,
+                                      int64_t y_bs, int64_t y_rs) {
+    if (geom == 1) return launch_lookback_geom<T, 1, STD, FUSEDT, BLOCK>(p, maps, grid, st, y, y_bs, y_rs);
+    if (geom == 2) return launch_lookback_geom<T, 2, STD, FUSEDT, BLOCK>(p, maps, grid, st, y, y_bs, y_rs);
+    return launch_lookback_geom<T, 0, STD, FUSEDT, BLOCK>(p, maps, grid, st, y, y_bs, y_rs);
 }
 
-// 1: the fused dt projection of the block's one-lane-per-channel scan runs as tcgen05.mma into tensor memory; 0: as
-// mma.sync in the producer warp, through a shared-memory tile.
-#ifndef HX_SCAN_FUSEDT_TC
-#define HX_SCAN_FUSEDT_TC 1
-#endif
 // ring stages of that form: with two, the chain load -> MMA -> commit of the next chunk does not always fit under the
 // 16 steps of the current one (10.90 against 10.74 ms over the 24 blocks of the byte LM)
 // chained segments: split until the grid is about this many waves of CTA slots (measured at 49 152 chains with the
-// dt projection inside, per 24 blocks: 3 waves = 4 segments 10.98 ms, 6 = 8 segments 10.7-10.8, 12 = 16 segments 11.08)
+// dt projection inside, us a launch: 4 segments 404, 6 392, 7 394, 8 389, 16 398)
 #ifndef HX_SCAN_CHAIN_WAVES
-#define HX_SCAN_CHAIN_WAVES 6.0
+#define HX_SCAN_CHAIN_WAVES 7.0
 #endif
 #ifndef HX_SCAN_FUSEDT_STAGES
 #define HX_SCAN_FUSEDT_STAGES 3
@@ -984,9 +986,9 @@ static int choose_cpl(const hx_scan_args *a) {
     return chains / 64.0 >= HX_SCAN_CPL2_MIN_WARPS * sm_count() ? 2 : 1;
 }
 
-// What the look-back form supports: geometric A, and where the dt projection is fused the block's configuration.
+// What the look-back form supports: d_state 16, and where the dt projection is fused the block's configuration.
 static bool lookback_ok(const hx_scan_args *a) {
-    if (a->d_state != 16 || !a->a_geometric || a->z_is_gate) return false;
+    if (a->d_state != 16 || a->z_is_gate) return false;
     if (a->W_dt) return a->conv_w == nullptr && a->z != nullptr && a->dt_softplus != 0;
     return true;
 }
@@ -1001,12 +1003,12 @@ static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t s
     const int ES = bf ? 2 : 4, BOXC = 128 / ES, TC = 16;
     if (form == 1)
         HX_REQUIRE(lookback_ok(a), HX_ERR_UNSUPPORTED_OPERATION,
-                   "the look-back scan needs a_geometric = 1 (and, with a fused dt projection, the block's configuration)");
+                   "the look-back scan takes raw z and, with a fused dt projection, the block's configuration");
     const int cpl = form == 1 ? 1 : choose_cpl(a);
     const int DT = bf ? (cpl == 2 ? 256 : 128) : 128;  // channels per CTA (4 consumer warps)
     const int tiles = (a->d_inner + DT - 1) / DT;
     int n_seg = 1, seg_len = (a->seq_len + TC - 1) / TC * TC;
-    if (split) seg_plan(a, kPlanChunk, &n_seg, &seg_len);
+    if (split) seg_plan(a, form == 1 ? TC : kPlanChunk, &n_seg, &seg_len);
     if (n_seg <= 1) form = 0;
 
     TiledParams p;
@@ -1081,28 +1083,30 @@ static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t s
     HX_REQUIRE(a->batch <= 65535 && n_seg <= 65535, HX_ERR_INVALID_DIMENSION, "batch %d or segments %d exceed the grid limit",
                a->batch, n_seg);
     dim3 grid(tiles, a->batch, n_seg - p.seg_base);
-    const bool geom = a->a_geometric != 0;
+    const int geom = a->a_geometric == 2 ? 2 : a->a_geometric != 0;
     const bool stdp = a->conv_w != nullptr && a->z != nullptr && a->dt_softplus != 0;
-    // the block's own call: u already convolved, gate and softplus present, geometric A
-    const bool blockp = bf && geom && !p.z_gate && a->conv_w == nullptr && a->z != nullptr && a->dt_softplus != 0;
+    // the block's own call: u already convolved, gate and softplus present
+    const bool blockp = bf && !p.z_gate && a->conv_w == nullptr && a->z != nullptr && a->dt_softplus != 0;
     void *yv = a->y;
     const int64_t ybs = a->y_batch_stride, yrs = a->y_row_stride;
     if (form == 1) {
-        if (fused_dt) {
-            if (HX_SCAN_FUSEDT_TC) return launch_lookback_pair<__nv_bfloat16, false, 2, true>(p, maps, grid, st, yv, ybs, yrs);
-            return launch_lookback_pair<__nv_bfloat16, false, 1, true>(p, maps, grid, st, yv, ybs, yrs);
-        }
-        if (blockp) return launch_lookback_pair<__nv_bfloat16, false, 0, true>(p, maps, grid, st, yv, ybs, yrs);
-        if (bf && stdp) return launch_lookback_pair<__nv_bfloat16, true, 0, false>(p, maps, grid, st, yv, ybs, yrs);
-        if (bf) return launch_lookback_pair<__nv_bfloat16, false, 0, false>(p, maps, grid, st, yv, ybs, yrs);
-        return launch_lookback_pair<float, false, 0, false>(p, maps, grid, st, yv, ybs, yrs);
+        if (fused_dt) return launch_lookback_pair<__nv_bfloat16, false, 2, true>(geom, p, maps, grid, st, yv, ybs, yrs);
+        if (blockp) return launch_lookback_pair<__nv_bfloat16, false, 0, true>(geom, p, maps, grid, st, yv, ybs, yrs);
+        if (bf && stdp) return launch_lookback_pair<__nv_bfloat16, true, 0, false>(geom, p, maps, grid, st, yv, ybs, yrs);
+        if (bf) return launch_lookback_pair<__nv_bfloat16, false, 0, false>(geom, p, maps, grid, st, yv, ybs, yrs);
+        return launch_lookback_pair<float, false, 0, false>(geom, p, maps, grid, st, yv, ybs, yrs);
     }
+// one instantiation per form of A
+#define HX_DIRECT_GEOM(T, CPL, STD, ...)                                                                               \
+    do {                                                                                                               \
+        if (geom == 1) return launch_direct_inst<T, CPL, 1, STD, ##__VA_ARGS__>(p, maps, grid, st, yv, ybs, yrs);      \
+        if (geom == 2) return launch_direct_inst<T, CPL, 2, STD, ##__VA_ARGS__>(p, maps, grid, st, yv, ybs, yrs);      \
+        return launch_direct_inst<T, CPL, 0, STD, ##__VA_ARGS__>(p, maps, grid, st, yv, ybs, yrs);                     \
+    } while (0)
 #define HX_DIRECT_CASE(T, CPL)                                                                                         \
     do {                                                                                                               \
-        if (geom && stdp) return launch_direct_inst<T, CPL, true, true>(p, maps, grid, st, yv, ybs, yrs);              \
-        if (geom) return launch_direct_inst<T, CPL, true, false>(p, maps, grid, st, yv, ybs, yrs);                     \
-        if (stdp) return launch_direct_inst<T, CPL, false, true>(p, maps, grid, st, yv, ybs, yrs);                     \
-        return launch_direct_inst<T, CPL, false, false>(p, maps, grid, st, yv, ybs, yrs);                              \
+        if (stdp) HX_DIRECT_GEOM(T, CPL, true);                                                                        \
+        HX_DIRECT_GEOM(T, CPL, false);                                                                                 \
     } while (0)
     if (fused_dt) {
         HX_REQUIRE(stdp || (a->z != nullptr && a->dt_softplus != 0), HX_ERR_UNSUPPORTED_OPERATION,
@@ -1111,60 +1115,86 @@ static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t s
         // the gate flag is a compile-time constant on this path (the block's), so the activation code is gone when
         // in_proj has already applied it
         if (p.z_gate) {
-            if (cpl == 2) {
-                if (geom) return launch_direct_inst<__nv_bfloat16, 2, true, false, 2, 1, true>(p, maps, grid, st, yv, ybs, yrs);
-                return launch_direct_inst<__nv_bfloat16, 2, false, false, 2, 1, true>(p, maps, grid, st, yv, ybs, yrs);
-            }
-            if (geom) return launch_direct_inst<__nv_bfloat16, 1, true, false, 2, 1, true>(p, maps, grid, st, yv, ybs, yrs);
-            return launch_direct_inst<__nv_bfloat16, 1, false, false, 2, 1, true>(p, maps, grid, st, yv, ybs, yrs);
+            if (cpl == 2) HX_DIRECT_GEOM(__nv_bfloat16, 2, false, 2, 1, true);
+            HX_DIRECT_GEOM(__nv_bfloat16, 1, false, 2, 1, true);
         }
         // the block's own call: every flag is a compile-time constant, which saves the per-point flag tests and the
         // registers of the unused conv window
         if (blockp) {
-            if (cpl == 2) return launch_direct_inst<__nv_bfloat16, 2, true, false, 2, 1, false, true>(p, maps, grid, st, yv, ybs, yrs);
+            if (cpl == 2) HX_DIRECT_GEOM(__nv_bfloat16, 2, false, 2, 1, false, true);
             // one lane per channel: the projection runs as tcgen05.mma into tensor memory, lane = channel
-            if (HX_SCAN_FUSEDT_TC)
-                return launch_direct_inst<__nv_bfloat16, 1, true, false, HX_SCAN_FUSEDT_STAGES, 2, false, true>(p, maps, grid, st, yv, ybs, yrs);
-            return launch_direct_inst<__nv_bfloat16, 1, true, false, 2, 1, false, true>(p, maps, grid, st, yv, ybs, yrs);
+            HX_DIRECT_GEOM(__nv_bfloat16, 1, false, HX_SCAN_FUSEDT_STAGES, 2, false, true);
         }
-        if (cpl == 2) {
-            if (geom) return launch_direct_inst<__nv_bfloat16, 2, true, false, 2, 1>(p, maps, grid, st, yv, ybs, yrs);
-            return launch_direct_inst<__nv_bfloat16, 2, false, false, 2, 1>(p, maps, grid, st, yv, ybs, yrs);
-        }
-        if (geom) return launch_direct_inst<__nv_bfloat16, 1, true, false, 2, 1>(p, maps, grid, st, yv, ybs, yrs);
-        return launch_direct_inst<__nv_bfloat16, 1, false, false, 2, 1>(p, maps, grid, st, yv, ybs, yrs);
+        if (cpl == 2) HX_DIRECT_GEOM(__nv_bfloat16, 2, false, 2, 1);
+        HX_DIRECT_GEOM(__nv_bfloat16, 1, false, 2, 1);
     }
-    if (bf && geom && stdp && a->reserved / 10 == 1) {  // tuning: three stages instead of two
-        if (cpl == 2) return launch_direct_inst<__nv_bfloat16, 2, true, true, 3>(p, maps, grid, st, yv, ybs, yrs);
-        return launch_direct_inst<__nv_bfloat16, 1, true, true, 3>(p, maps, grid, st, yv, ybs, yrs);
+    if (bf && geom == 1 && stdp && a->reserved / 10 == 1) {  // tuning: three stages instead of two
+        if (cpl == 2) return launch_direct_inst<__nv_bfloat16, 2, 1, true, 3>(p, maps, grid, st, yv, ybs, yrs);
+        return launch_direct_inst<__nv_bfloat16, 1, 1, true, 3>(p, maps, grid, st, yv, ybs, yrs);
     }
     if (blockp) {
         // the block's configuration with dt read from memory: compile-time flags as in the fused form
-        if (cpl == 2) return launch_direct_inst<__nv_bfloat16, 2, true, false, 2, 0, false, true>(p, maps, grid, st, yv, ybs, yrs);
-        return launch_direct_inst<__nv_bfloat16, 1, true, false, 2, 0, false, true>(p, maps, grid, st, yv, ybs, yrs);
+        if (cpl == 2) HX_DIRECT_GEOM(__nv_bfloat16, 2, false, 2, 0, false, true);
+        HX_DIRECT_GEOM(__nv_bfloat16, 1, false, 2, 0, false, true);
     }
     if (bf) {
         if (cpl == 2) HX_DIRECT_CASE(__nv_bfloat16, 2);
         HX_DIRECT_CASE(__nv_bfloat16, 1);
     }
     HX_DIRECT_CASE(float, 1);
+#undef HX_DIRECT_GEOM
 #undef HX_DIRECT_CASE
     return HX_OK;
 }
 
 // ---- kernel choice of HX_SCAN_AUTO (d_state == 16), shared with the Mamba block's planning
-// Chains are (batch, channel) pairs; a one-lane-per-channel warp holds 32 of them.  With at least 8 such warps per
-// SM the direct kernel runs them one pass, chained segments evening out the load.  Below that the machine is short
-// of independent work: with geometric A and a split the look-back form runs the segments of a chain at the same
-// time; otherwise the lane-split kernel spreads a chain's states over 2 or 4 lanes.
+// Chains are (batch, channel) pairs; a one-lane-per-channel warp holds 32 of them.  A warp scheduler is as good as full
+// with ONE such bf16 warp (158 cycles a step alone, 142 to 144 a step and warp with two or three: the fp32x2 operands
+// saturate the register ports), so one pass over the sequence beats the look-back form, which does 1.25 to 1.5 x the
+// work, from about 2.5 warps per SM on.  Measured, us, one pass / look-back: [16, 4096, 1536] 515 / 612, [16, 2048, 1536]
+// 272 / 317, [12, 1024, 2048] 146 / 165, [6, 1500, 2048] 127 / 131 (general A 215 / 203), [10, 2000, 1024] 166 / 144.  The
+// fp32 form is bound by the latency of its accurate exp, log and division chains (550 cycles a step alone) and gains from
+// a second warp: [12, 1024, 2048] 348 / 365, [6, 1500, 2048] 447 / 277.
+static double warps_per_sm(const hx_scan_args *a) { return (double)a->batch * a->d_inner / 32.0 / sm_count(); }
+static bool one_pass_pays(const hx_scan_args *a) {
+    const double limit = a->io_dtype != HX_BF16 ? 4.0 : a->a_geometric == 1 ? 2.5 : 3.0;
+    return warps_per_sm(a) >= limit;
+}
+// Sequences this short are over before a second launch starts: one pass (bf16) or the lane-split kernel (fp32, general A).
+// Measured at 1 x 100 x 1536: bf16 12.5 us in one pass; fp32 18.7 us lane-split against 25 us in the look-back form.
+static bool short_sequence(const hx_scan_args *a) { return a->seq_len < (a->io_dtype == HX_BF16 ? 64 : 192); }
+
 int auto_channels_per_lane(const hx_scan_args *a) { return choose_cpl(a); }
 
 ScanKind auto_kind(const hx_scan_args *a) {
-    const double warps_per_sm = (double)a->batch * a->d_inner / 32.0 / sm_count();
-    if (warps_per_sm >= 8.0) return ScanKind::Direct;
+    if (one_pass_pays(a)) return ScanKind::Direct;
     if (a->seq_splits > 1 && lookback_ok(a)) return ScanKind::LookBack;
     if (a->W_dt != nullptr) return ScanKind::Direct;  // the fused dt projection exists only there
+    if (a->io_dtype == HX_BF16 && a->a_geometric != 0) return ScanKind::Direct;
     return ScanKind::Tiled;
+}
+
+// Sequence segments for AUTO.
+int auto_splits(const hx_scan_args *a) {
+    if (!one_pass_pays(a) && !a->z_is_gate) {
+        // look-back form: as many segments as fill the three CTAs an SM holds once (one more and some SMs run a fourth
+        // after the others: [3, 1631, 1536] with 10 / 16 segments 3.39 / 3.28 ms a model pass, 12 fill 432 of 444 slots), of
+        // at least 32 steps (16 where the sequence has few)
+        if (short_sequence(a)) return 1;
+        const int by_length = a->seq_len / (a->seq_len < 160 ? 16 : 32);
+        int s = 3 * sm_count() / (a->batch * ((a->d_inner + 127) / 128));
+        if (s > by_length) s = by_length;
+        return s < 1 ? 1 : s > 32 ? 32 : s;
+    }
+    // Chained segments even out CTAs that do not fill the SMs equally; nothing to even out below one CTA (4 warps) per SM
+    // or far above the slots of the device (about 3 CTAs per SM), and the fp32 form only loses by the hand-overs.
+    const int tile = one_pass_pays(a) ? 128 : (a->io_dtype == HX_BF16 ? 64 : 32);
+    const double ctas = (double)a->batch * ((a->d_inner + tile - 1) / tile), slots = 3.0 * sm_count();
+    if (ctas >= 8.0 * slots || ctas <= sm_count() || (a->io_dtype != HX_BF16 && one_pass_pays(a))) return 1;
+    int s = (int)(HX_SCAN_CHAIN_WAVES * slots / ctas + 0.999);
+    if (s > 8) s = 8;                                      // 8 segments: within 2 % of the best at every shape measured
+    if (s > a->seq_len / 160) s = a->seq_len / 160;        // a hand-over costs about 2 us
+    return s < 1 ? 1 : s;
 }
 
 }  // namespace scan
@@ -1193,7 +1223,9 @@ hx_status hx_selective_scan_fwd(const hx_scan_args *a, void *stream) {
         case HX_SCAN_TILED: return hx::scan::launch_tiled(a, split, st);
         case HX_SCAN_SEQSPLIT: return hx::scan::launch_tiled(a, true, st);
         case HX_SCAN_DIRECT: return hx::scan::launch_direct(a, split, st);
-        case HX_SCAN_LOOKBACK: return hx::scan::launch_direct(a, true, st, 1);
+        case HX_SCAN_LOOKBACK:
+            HX_REQUIRE(a->a_geometric, HX_ERR_UNSUPPORTED_OPERATION, "HX_SCAN_LOOKBACK needs a_geometric (HX_SCAN_AUTO takes any A)");
+            return hx::scan::launch_direct(a, true, st, 1);
         case HX_SCAN_AUTO: {
             if (a->d_state == 16) {
                 switch (hx::scan::auto_kind(a)) {
@@ -1212,28 +1244,7 @@ hx_status hx_selective_scan_fwd(const hx_scan_args *a, void *stream) {
 
 int32_t hx_selective_scan_suggest_splits(const hx_scan_args *a) {
     if (!a || a->d_state != 16 || a->batch <= 0 || a->seq_len <= 0 || a->d_inner <= 0) return 1;
-    const double chains = (double)a->batch * a->d_inner;
-    const double warps_per_sm = chains / 32.0 / hx::sm_count();
-    const bool direct = warps_per_sm >= 8.0;
-    if (!direct && a->a_geometric && !a->z_is_gate) {
-        // few chains, geometric A: the look-back form runs the segments of a chain at the same time.  Its aggregate
-        // pass covers all segments but the last, so split until that pass alone has about 8 one-lane-per-channel
-        // warps per SM (measured: below that it is short of warps, beyond it the extra work of shorter segments
-        // buys nothing), keeping segments of at least 64 steps
-        int splits = 1;
-        while (splits < 16 && (splits - 1) * warps_per_sm < 8.0 && a->seq_len / (2 * splits) >= 64) splits *= 2;
-        return splits;
-    }
-    // chained segments: CTAs of the kernel AUTO would pick, against the CTA slots of the device (about 3 per SM)
-    const int tile = direct ? 128 : (a->io_dtype == HX_BF16 ? 64 : 32);
-    const double ctas = (double)a->batch * ((a->d_inner + tile - 1) / tile);
-    const double slots = 3.0 * hx::sm_count();
-    if (ctas >= 8.0 * slots) return 1;
-    int want = (int)(HX_SCAN_CHAIN_WAVES * slots / ctas + 0.999);
-    int splits = 1;
-    while (splits < want && splits < 16) splits *= 2;
-    while (splits > 1 && a->seq_len / splits < 128) splits /= 2;  // keep segments long enough to amortise the hand-over
-    return splits;
+    return hx::scan::auto_splits(a);
 }
 
 hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *a, size_t *bytes) {
@@ -1242,7 +1253,9 @@ hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *a, size_t *bytes
     if (a->variant != HX_SCAN_SEQSPLIT && a->variant != HX_SCAN_LOOKBACK && a->seq_splits <= 1) return HX_OK;
     if (a->variant == HX_SCAN_SIMPLE) return HX_OK;
     int n_seg, seg_len;
-    hx::scan::seg_plan(a, hx::scan::kPlanChunk, &n_seg, &seg_len);
+    // the finer plan has the most segments, so the size serves every form the variant may run
+    const bool may_look_back = a->variant == HX_SCAN_AUTO || a->variant == HX_SCAN_LOOKBACK;
+    hx::scan::seg_plan(a, may_look_back ? 16 : hx::scan::kPlanChunk, &n_seg, &seg_len);
     *bytes = hx::scan::workspace_bytes(a, n_seg);
     return HX_OK;
 }

@@ -64,7 +64,7 @@ def scan_workspace_bytes(batch, seq_len, d_inner, dtype, seq_splits=0) -> int:
     a = L.ScanArgs()
     a.batch, a.seq_len, a.d_inner, a.d_state = batch, seq_len, d_inner, 16
     a.io_dtype = L.HX_BF16 if dtype == torch.bfloat16 else L.HX_F32
-    a.variant = L.SCAN_SEQSPLIT
+    a.variant = L.SCAN_LOOKBACK  # the largest of the split forms
     a.seq_splits = seq_splits
     n = C.c_size_t(0)
     L.check(L.lib().hx_selective_scan_workspace_bytes(C.byref(a), C.byref(n)))
@@ -84,7 +84,9 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, d
                    variant=L.SCAN_AUTO, a_geometric=None, lanes_per_channel=0, return_state=False, out=None,
                    workspace=None, seq_splits=0, tune=0, dt_low=None, W_dt=None, z_is_gate=False):
     """Fused selective scan (hx_selective_scan_fwd).  x, dt, z, y: [B, L, D]; Bm, Cm: [B, L, N].
-    z_is_gate: z already holds silu(z)."""
+    z_is_gate: z already holds silu(z).
+    With every choice left open (SCAN_AUTO, seq_splits 0) the library plans the sequence segments, and a_geometric=None
+    leaves it to the kernel to look at A: no device-to-host copy, no synchronisation."""
     Bsz, Lq, Dm = x.shape
     N = A.shape[1]
     y = out if out is not None else torch.empty((Bsz, Lq, Dm), dtype=x.dtype, device=x.device)
@@ -126,17 +128,22 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, d
             setattr(a, name, _f32(t).data_ptr())
     if h is not None:
         a.h_last = h.data_ptr()
-    if a_geometric is None:
-        a_geometric = check_geometric(A)
-    a.a_geometric = 1 if a_geometric else 0
-    a.lanes_per_channel = lanes_per_channel
-    a.seq_splits = seq_splits
-    a.reserved = tune
     a.z_is_gate = 1 if z_is_gate else 0
+    a.lanes_per_channel = lanes_per_channel
+    a.reserved = tune
+    auto = variant == L.SCAN_AUTO
+    if a_geometric is None:
+        a.a_geometric = 2 if auto and N == 16 else (1 if check_geometric(A) else 0)
+    else:
+        a.a_geometric = 1 if a_geometric else 0
+    planned = auto and seq_splits == 0 and N == 16 and Bsz > 0 and Lq > 0 and Dm > 0
+    if planned:
+        seq_splits = int(L.lib().hx_selective_scan_suggest_splits(C.byref(a)))
+    a.seq_splits = seq_splits
     if variant in (L.SCAN_SEQSPLIT, L.SCAN_LOOKBACK) or seq_splits > 1:
         n = C.c_size_t(0)
         L.check(L.lib().hx_selective_scan_workspace_bytes(C.byref(a), C.byref(n)))
-        if workspace is None:
+        if workspace is None or (planned and workspace.numel() * workspace.element_size() < n.value):
             workspace = torch.empty(max(n.value, 1), dtype=torch.uint8, device=x.device)
         a.workspace = workspace.data_ptr()
         a.workspace_bytes = workspace.numel() * workspace.element_size()
@@ -305,9 +312,10 @@ def mamba_block(x, w: dict, d_state: int, d_conv: int, workspace=None, scan_vari
     a.Dskip = _f32(w["D"]).data_ptr()
     # the scan's plan (and with it the workspace size) depends on the variant and on whether A is geometric
     a.scan_variant = scan_variant
-    if a_geometric is None:
-        a_geometric = check_geometric(w["A"])
-    a.a_geometric = 1 if a_geometric else 0
+    if a_geometric is None and scan_variant == L.SCAN_AUTO and d_state == 16:
+        a.a_geometric = 2  # the kernel looks at A itself: no copy back, no synchronisation
+    else:
+        a.a_geometric = 1 if (check_geometric(w["A"]) if a_geometric is None else a_geometric) else 0
     n = C.c_size_t(0)
     L.check(L.lib().hx_mamba_block_workspace_bytes(C.byref(a), C.byref(n)))
     if workspace is None:

@@ -135,11 +135,13 @@ typedef struct hx_scan_args {
                                  `workspace`).  HX_SCAN_TILED / DIRECT: in order, each starting from its
                                  predecessor's final state, which evens out the load when batch * d_inner / tile
                                  is not a multiple of the SM slots.  HX_SCAN_LOOKBACK: at the same time.
-                                 HX_SCAN_AUTO: chained when chains are plentiful, look-back when they are few and
-                                 A is geometric.  HX_SCAN_SEQSPLIT / LOOKBACK: 0 = four segments */
+                                 HX_SCAN_AUTO: chained when chains are plentiful, look-back (for any A) when they are
+                                 few.  HX_SCAN_SEQSPLIT / LOOKBACK: 0 = four segments */
     int32_t a_geometric;      /* 1: the caller asserts A[d][n] == (n+1) * A[d][0] (checked once with
                                  hx_scan_check_geometric); then exp(dt*A[d][n]) is evaluated as a power of
-                                 exp(dt*A[d][0]), one exp per point instead of d_state */
+                                 exp(dt*A[d][0]), one exp per point instead of d_state.  0: a general A.  2: not known to
+                                 the caller; the one-lane-per-channel kernel looks at the A rows of its channels itself
+                                 (the other kernels treat 2 as 0) */
     int32_t lanes_per_channel;/* HX_SCAN_TILED / SEQSPLIT: lanes that share one channel's 16 states
                                  (1, 2 or 4; 0 = choose from the problem size) */
     int32_t reserved;         /* tuning selector, 0 = default.  HX_SCAN_DIRECT: channels per lane (1 or 2) */
@@ -163,9 +165,9 @@ HX_API hx_status hx_selective_scan_fwd(const hx_scan_args *args, void *stream);
 /* Bytes of `workspace` a split scan of these dimensions needs (HX_SCAN_SEQSPLIT, HX_SCAN_LOOKBACK, or any variant
  * with seq_splits > 1; 0 otherwise).  One size serves the chained and the look-back form. */
 HX_API hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *args, size_t *bytes);
-/* Number of sequence segments (a power of two, 1 = do not split) HX_SCAN_AUTO works best with for these dimensions
+/* Number of sequence segments (1 = do not split) HX_SCAN_AUTO works best with for these dimensions
  * on the current device: chained segments that even out the load when chains are plentiful, parallel segments
- * (look-back form, needs args->a_geometric) when they are few.  Pass it as args->seq_splits with a workspace. */
+ * (look-back form) when they are few.  Pass it as args->seq_splits with a workspace. */
 HX_API int32_t hx_selective_scan_suggest_splits(const hx_scan_args *args);
 /* The same operation on HOST activations: x, dt, z, Bm, Cm are read from (preferably pinned) host memory
  * with the strides given in args, staged into `dev_workspace` (caller-owned device memory of

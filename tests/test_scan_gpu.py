@@ -523,3 +523,35 @@ def test_gather_push_places_shards_at_their_columns():
     assert _lib.lib().hx_allgather_y_push(C.byref(a), st) == 5
     a.col0, a.world = 128, 9
     assert _lib.lib().hx_allgather_y_push(C.byref(a), st) == 10
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("L,splits", [(33, 2), (200, 5), (700, 16)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_auto_lookback_general_decay(dtype, L, splits, mixed):
+    """Few chains and a general A: AUTO's look-back form (ragged last segment, more segments than one batch of folded
+    aggregates).  mixed: the first 128 channels are geometric, so that with a_geometric left open the CTAs of one launch
+    take different forms."""
+    inp = synth.scan_inputs(61, 2, L, 160, 16, 4, bf16=dtype == "bf16")
+    inp["A"] = -np.exp(synth.uniform(61, "Alog", (160, 16), -1.0, 2.0)).astype(np.float32)
+    if mixed:
+        inp["A"][:128] = -np.arange(1, 17, dtype=np.float32)
+    inp["dt"] = inp["dt"] - 2.0
+    if dtype == "bf16":
+        inp["dt"] = synth.round_bf16(inp["dt"])
+    ref, hr = run_ref(inp, state=True)
+    for geom in (None, False):
+        got, hg = run_gpu(inp, dtype, variant=0, geom=geom, seq_splits=splits, state=True)
+        check_blocks(got, ref, dtype, 16)
+        check(hg, hr, dtype)
+
+
+@pytest.mark.parametrize("L", [63, 64, 191, 192, 400])
+def test_auto_plans_segments_of_default_calls(L):
+    """Every choice left to the library, on both sides of the lengths where its plan changes."""
+    for dtype in ("f32", "bf16"):
+        inp = synth.scan_inputs(62, 1, L, 96, 16, 4, bf16=dtype == "bf16")
+        got, hg = run_gpu(inp, dtype, variant=0, state=True)
+        ref, hr = run_ref(inp, state=True)
+        check_blocks(got, ref, dtype, 32)
+        check(hg, hr, dtype)
