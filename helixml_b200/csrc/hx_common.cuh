@@ -63,6 +63,7 @@ namespace scan {
 enum class ScanKind { Tiled, Direct, LookBack };
 ScanKind auto_kind(const hx_scan_args *a);
 int auto_channels_per_lane(const hx_scan_args *a);  // 1 or 2: what the one-lane-per-channel kernel would run with
+hx_status launch_wide(const hx_scan_args *a, cudaStream_t st);  // any d_state and alignment (scan_wide.cu); a validated
 }  // namespace scan
 
 // Translation units with bounded device-side waits keep a status word each; these read (and

@@ -4,8 +4,9 @@
 //
 // Two kernels:
 //   scan_simple_kernel  one thread per (batch, channel), any d_state <= 256, accurate libm-style
-//                       math.  The parity baseline and the fallback for shapes the tiled kernel
-//                       does not take.
+//                       math.  The parity baseline (HX_SCAN_SIMPLE).
+//                       HX_SCAN_AUTO runs scan_wide_kernel (scan_wide.cu) for the shapes the other
+//                       kernels do not take.
 //   scan_tiled_kernel   d_state == 16.  A CTA owns one batch row and a 128-byte-wide channel tile
 //                       and walks the sequence in chunks.  A producer warp moves [chunk x tile]
 //                       boxes of x/dt/z/B/C into shared memory with TMA (3-D tensor maps, 128-byte
@@ -1233,10 +1234,10 @@ hx_status hx_selective_scan_fwd(const hx_scan_args *a, void *stream) {
                     case hx::scan::ScanKind::LookBack: s = hx::scan::launch_direct(a, true, st, 1); break;
                     default: s = hx::scan::launch_tiled(a, split, st); break;
                 }
-                // an operand that does not meet the TMA alignment rules goes to the simple kernel
+                // an operand that does not meet the TMA alignment rules goes to the general kernel
                 if (s != HX_ERR_UNSUPPORTED_OPERATION) return s;
             }
-            return hx::scan::launch_simple(a, st);
+            return hx::scan::launch_wide(a, st);
         }
         default: return hx::fail(HX_ERR_INVALID_INPUT, "unknown scan variant %d", a->variant);
     }

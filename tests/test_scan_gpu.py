@@ -59,6 +59,24 @@ def check_blocks(got, ref, dtype, seg_len, tile=64):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("d_state,seq_len,d_inner", [(1, 1, 1), (8, 15, 33), (9, 16, 31), (16, 17, 9), (17, 32, 16), (32, 33, 17),
+                                                     (33, 47, 8), (64, 49, 9), (65, 31, 8), (128, 18, 7), (129, 20, 4), (256, 35, 5)])
+def test_wide_kernel(dtype, d_state, seq_len, d_inner):
+    """Every lane split, ragged channel tiles and chunks, with and without conv, gate and skip (d_state 16 with an odd
+    d_inner: operands that miss the alignment rules of the other kernels)."""
+    inp = synth.scan_inputs(71, 2, seq_len, d_inner, d_state, 4, bf16=dtype == "bf16")
+    got, hg = run_gpu(inp, dtype, variant=0, geom=False, state=True)
+    ref, hr = run_ref(inp, state=True)
+    check(got, ref, dtype)
+    assert fp32_tol_err(hg, hr) <= FP32_TOL
+    # dt is drawn for softplus (negative); used as it is it must be positive: a step with dt < 0 grows a state by
+    # exp(|dt| d_state), up to e^1000 here, and the oracle overflows as well
+    inp["dt"] = -inp["dt"] / 8
+    check(run_gpu(inp, dtype, variant=0, geom=False, gate=False, skip=False, conv=False, softplus=False),
+          run_ref(inp, gate=False, skip=False, conv=False, softplus=False), dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_simple_kernel(dtype):
     inp = synth.scan_inputs(31, 2, 50, 40, 16, 4, bf16=dtype == "bf16")
     got, hg = run_gpu(inp, dtype, variant=SIMPLE, state=True)
