@@ -151,30 +151,84 @@ s4_diag_kernel(const T *u, const float *A, const float *Bp, const float *Cp, con
 
 // ---------------------------------------------------------------- reference-literal S4
 // V[t][n] = sum_m (dt * B[n][m]) * u[m][t]   (m ascending, as the reference's matvec)
+//
+// The three kernels below are small (forward_ssm at d_model 256, 2048 steps, 64 states: 67 M FMA, 4.5 MB), so what counts
+// is latency: enough CTAs, a register tile per thread so that an operand read from shared memory serves several
+// products, and the next slab's global loads in flight under the current one.  Every output keeps one accumulator over
+// ascending m (n), so the sums are those of a thread-per-output loop bit for bit.  At that shape, in us, as one
+// thread per output with operands from global memory -> now: in 21.9 -> 10.1, scan (one CTA for all states) 31.7 -> 7.5,
+// out 125.4 -> 6.0; the whole call, host array to host array, 485 -> 315.
+constexpr int kRT = 32;  // tile of steps
+constexpr int kRN = 32;  // tile of states (s4_ref_in), slab of the summed index
+constexpr int kRM = 64;  // tile of channels (s4_ref_out)
+
+// CTA: 32 steps x 32 states, thread: 2 steps x 4 states.
 __global__ void __launch_bounds__(128)
 s4_ref_in_kernel(const float *u, const float *Bm, float dt, float *V, int M, int L, int N) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = blockIdx.y;
-    if (t >= L) return;
-    float sum = 0.f;
-    for (int m = 0; m < M; ++m) sum += (Bm[(int64_t)n * M + m] * dt) * u[(int64_t)m * L + t];
-    V[(int64_t)t * N + n] = sum;
+    __shared__ __align__(16) float us[kRN][kRT], bs[kRN][kRN + 4];  // [m][t], [m][n]
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int t0 = blockIdx.x * kRT, n0 = blockIdx.y * kRN;
+    float ur[8], br[8];
+    auto fetch = [&](int m0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int i = tid + k * 128, lo = i % 32, hi = i / 32;
+            ur[k] = (m0 + hi < M && t0 + lo < L) ? u[(int64_t)(m0 + hi) * L + t0 + lo] : 0.f;
+            br[k] = (n0 + hi < N && m0 + lo < M) ? Bm[(int64_t)(n0 + hi) * M + m0 + lo] : 0.f;
+        }
+    };
+    float acc[2][4] = {};
+    fetch(0);
+    for (int m0 = 0; m0 < M; m0 += kRN) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int i = tid + k * 128, lo = i % 32, hi = i / 32;
+            us[hi][lo] = ur[k];
+            bs[lo][hi] = br[k] * dt;
+        }
+        __syncthreads();
+        if (m0 + kRN < M) fetch(m0 + kRN);
+        const int mn = min(kRN, M - m0);
+#pragma unroll 8
+        for (int m = 0; m < mn; ++m) {
+            const float2 uv = *reinterpret_cast<const float2 *>(&us[m][tx * 2]);
+            const float4 bv = *reinterpret_cast<const float4 *>(&bs[m][ty * 4]);
+            const float b4[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[0][j] = fmaf(b4[j], uv.x, acc[0][j]);
+                acc[1][j] = fmaf(b4[j], uv.y, acc[1][j]);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int t = t0 + tx * 2 + i, n = n0 + ty * 4 + j;
+            if (t < L && n < N) V[(int64_t)t * N + n] = acc[i][j];
+        }
 }
 
 // In-place diagonal scan over time on V [L][N]: X_t = a X_{t-1} + V_t, a = exp(dt A_re) cos(dt A_im).
-// One CTA; thread = (state n, segment g); same 3-pass scheme through shared memory.
+// A CTA takes the kScanN states from blockIdx.x * kScanN on (their four-byte neighbours in a row make one 32-byte
+// sector); thread = (state, segment of the sequence); same 3-pass scheme through shared memory.
+constexpr int kScanN = 8;
 __global__ void __launch_bounds__(1024)
 s4_ref_scan_kernel(float *V, const float *A_real, const float *A_imag, float dt, int L, int N, int G) {
-    extern __shared__ float ends_s[];  // [G][N]
-    const int n = threadIdx.x % N, g = threadIdx.x / N;
-    const bool active = g < G;
+    __shared__ float ends_s[1024];  // [G][kScanN]
+    const int nl = threadIdx.x % kScanN, g = threadIdx.x / kScanN, n = blockIdx.x * kScanN + nl;
+    const bool active = n < N;
     const float a = active ? expf(A_real[n] * dt) * cosf(A_imag[n] * dt) : 0.f;
     const int seg_len = (L + G - 1) / G;
     const int t0 = min(L, g * seg_len), t1 = min(L, t0 + seg_len);
     float h = 0.f;
-    if (active)
+    if (active) {
+#pragma unroll 16
         for (int t = t0; t < t1; ++t) h = a * h + V[(int64_t)t * N + n];
-    if (active) ends_s[g * N + n] = h;
+    }
+    ends_s[threadIdx.x] = h;
     __syncthreads();
     if (!active) return;
     float aT = 1.f, base = a;  // a^seg_len by binary exponentiation (a may be negative)
@@ -183,25 +237,93 @@ s4_ref_scan_kernel(float *V, const float *A_real, const float *A_imag, float dt,
         base *= base;
     }
     h = 0.f;
-    for (int gp = 0; gp < g; ++gp) h = aT * h + ends_s[gp * N + n];
-    for (int t = t0; t < t1; ++t) {
+#pragma unroll 8
+    for (int gp = 0; gp < g; ++gp) h = aT * h + ends_s[gp * kScanN + nl];
+    int t = t0;
+    for (; t + 8 <= t1; t += 8) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = V[(int64_t)(t + e) * N + n];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            h = a * h + v[e];
+            V[(int64_t)(t + e) * N + n] = h;
+        }
+    }
+    for (; t < t1; ++t) {
         h = a * h + V[(int64_t)t * N + n];
         V[(int64_t)t * N + n] = h;
     }
 }
 
 // y[t][m] = sum_n C[m][n] X[t][n] + D[m] u[m][t]   (n ascending)
+// CTA: 32 steps x 64 channels, thread: 4 steps x 4 channels.
 __global__ void __launch_bounds__(128)
 s4_ref_out_kernel(const float *X, const float *Cm, const float *Dv, const float *u, float *y, int M, int L, int N) {
-    extern __shared__ float xs[];  // X[t][:]
-    const int t = blockIdx.y;
-    for (int n = threadIdx.x; n < N; n += blockDim.x) xs[n] = X[(int64_t)t * N + n];
-    __syncthreads();
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    float sum = 0.f;
-    for (int n = 0; n < N; ++n) sum += Cm[(int64_t)m * N + n] * xs[n];
-    y[(int64_t)t * M + m] = sum + Dv[m] * u[(int64_t)m * L + t];
+    __shared__ __align__(16) float cs[kRN][kRM + 4], xs[kRN][kRT + 4];  // [n][m], [n][t]
+    __shared__ float us[kRM][kRT + 1];                                   // [m][t]
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int t0 = blockIdx.y * kRT, m0 = blockIdx.x * kRM;
+    float cr[16], xr[8];
+    auto fetch = [&](int n0) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int i = tid + k * 128, lo = i % 32, hi = i / 32;
+            cr[k] = (m0 + hi < M && n0 + lo < N) ? Cm[(int64_t)(m0 + hi) * N + n0 + lo] : 0.f;
+            if (k < 8) xr[k] = (t0 + hi < L && n0 + lo < N) ? X[(int64_t)(t0 + hi) * N + n0 + lo] : 0.f;
+        }
+    };
+    fetch(0);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int i = tid + k * 128, lo = i % 32, hi = i / 32;
+        us[hi][lo] = (m0 + hi < M && t0 + lo < L) ? u[(int64_t)(m0 + hi) * L + t0 + lo] : 0.f;
+    }
+    float acc[4][4] = {};
+    for (int n0 = 0; n0 < N; n0 += kRN) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int i = tid + k * 128, lo = i % 32, hi = i / 32;
+            cs[lo][hi] = cr[k];
+            if (k < 8) xs[lo][hi] = xr[k];
+        }
+        __syncthreads();
+        if (n0 + kRN < N) fetch(n0 + kRN);
+        const int nn = min(kRN, N - n0);
+#pragma unroll 8
+        for (int n = 0; n < nn; ++n) {
+            const float4 cv = *reinterpret_cast<const float4 *>(&cs[n][tx * 4]);
+            const float4 xv = *reinterpret_cast<const float4 *>(&xs[n][ty * 4]);
+            const float c4[4] = {cv.x, cv.y, cv.z, cv.w}, x4[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(c4[j], x4[i], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int m = m0 + tx * 4 + j;
+        if (m >= M) continue;
+        const float dv = Dv[m];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(dv, us[tx * 4 + j][ty * 4 + i], acc[i][j]);
+    }
+    const bool row16 = m0 + tx * 4 + 4 <= M && M % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = t0 + ty * 4 + i;
+        if (t >= L) continue;
+        float *yp = y + (int64_t)t * M + m0 + tx * 4;
+        if (row16) {
+            *reinterpret_cast<float4 *>(yp) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (m0 + tx * 4 + j < M) yp[j] = acc[i][j];
+        }
+    }
 }
 
 template <typename T>
@@ -274,18 +396,19 @@ hx_status hx_s4_ref_forward_ssm(const float *u, const float *A_real, const float
                "hx_s4_ref_forward_ssm needs a workspace of %zu bytes (got %zu)", need, workspace_bytes);
     cudaStream_t st = (cudaStream_t)stream;
     float *V = static_cast<float *>(workspace);
-    s4_ref_in_kernel<<<dim3((seq_len + 127) / 128, d_state), 128, 0, st>>>(u, Bm, dt, V, d_model, seq_len, d_state);
+    s4_ref_in_kernel<<<dim3((seq_len + kRT - 1) / kRT, (d_state + kRN - 1) / kRN), 128, 0, st>>>(u, Bm, dt, V, d_model, seq_len,
+                                                                                              d_state);
     hx_status s = hx::check_launch("s4_ref_in_kernel");
     if (s != HX_OK) return s;
-    int G = 1024 / d_state;
-    if (G > 32) G = 32;
-    if (G > seq_len) G = seq_len;
-    if (G < 1) G = 1;
-    s4_ref_scan_kernel<<<1, G * d_state, (size_t)G * d_state * sizeof(float), st>>>(V, A_real, A_imag, dt, seq_len,
-                                                                                  d_state, G);
+    // segments of at least 8 steps, up to the 1024 threads of a CTA; the segment count is a multiple of 4 so that a
+    // CTA is whole warps
+    int G = (seq_len + 7) / 8;
+    G = (G + 3) / 4 * 4;
+    if (G > 1024 / kScanN) G = 1024 / kScanN;
+    s4_ref_scan_kernel<<<(d_state + kScanN - 1) / kScanN, G * kScanN, 0, st>>>(V, A_real, A_imag, dt, seq_len, d_state, G);
     if ((s = hx::check_launch("s4_ref_scan_kernel")) != HX_OK) return s;
-    s4_ref_out_kernel<<<dim3((d_model + 127) / 128, seq_len), 128, d_state * sizeof(float), st>>>(V, Cm, Dv, u, y, d_model,
-                                                                                                 seq_len, d_state);
+    s4_ref_out_kernel<<<dim3((d_model + kRM - 1) / kRM, (seq_len + kRT - 1) / kRT), 128, 0, st>>>(V, Cm, Dv, u, y, d_model,
+                                                                                           seq_len, d_state);
     return hx::check_launch("s4_ref_out_kernel");
 }
 

@@ -54,6 +54,12 @@ def test_s4_reference_literal(M, L, N):
     assert fp32_tol_err(to_np(got), ref) <= FP32_TOL
 
 
+@pytest.mark.parametrize("M,L,N", [(1, 1, 1), (31, 33, 7), (33, 31, 9), (65, 64, 32), (63, 1030, 33), (129, 95, 256)])
+def test_s4_reference_literal_tile_edges(M, L, N):
+    """Around the tiles of 32 steps, 32 states and 64 channels, and the segments of 8 or more steps of the scan."""
+    test_s4_reference_literal(M, L, N)
+
+
 def test_s4_reference_literal_golden(golden):
     from helixml_b200 import ops
     g = golden("s4_ref_small.npz")
