@@ -172,6 +172,22 @@ def test_gemm_simt_f32(M, N, K):
     assert fp32_tol_err(to_np(got), cbind.linear(a, w, b)) <= FP32_TOL
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("M,N,K", [(31, 33, 61), (33, 31, 64), (32, 32, 130), (700, 641, 35), (641, 700, 36), (1500, 1400, 9),
+                                   (1409, 1536, 24)])
+def test_gemm_simt_tiles(dtype, M, N, K):
+    """Every tile size of the CUDA-core GEMM (by the number of tiles the shape has), ragged edges, an inner dimension that is
+    not a multiple of four, and a C whose rows are not 16-byte aligned."""
+    import torch
+    from helixml_b200 import ops
+    a, w, b = synth.normal(63, "a", (M, K)), synth.normal(63, "w", (N, K), 0, 0.1), synth.normal(63, "b", (N,))
+    if dtype == "bf16":
+        a, w = synth.round_bf16(a), synth.round_bf16(w)
+    cast = "bf16" if dtype == "bf16" else None
+    got = ops.gemm(to_dev(a, cast), to_dev(w, cast), to_dev(b), tensor_cores=False, out_dtype=torch.float32)
+    assert fp32_tol_err(to_np(got), cbind.linear(a, w, b)) <= FP32_TOL
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (256, 256, 128), (1000, 3072, 768), (513, 80, 1536), (300, 1536, 48),
                                    (70, 768, 1536), (4096, 256, 768), (129, 136, 72)])
 def test_gemm_tcgen05_bf16(M, N, K):
