@@ -5,8 +5,8 @@
 // block of the byte LM); here the tile of u the conv produces in shared memory IS the GEMM's A operand, so u is
 // written once (the scan reads it) and never read back.
 //
-// One CTA per 128 consecutive steps of one sequence (64 where that leaves SMs idle), all channels, walked in blocks
-// of 64 channels:
+// One CTA per 128 consecutive steps of one sequence (64 where that leaves SMs idle, and then the channels of a tile shared
+// by the CTAs of a cluster), all channels, walked in blocks of 64 channels:
 //   warp 0      TMA producer: [131 steps x 64 channels] boxes of x (3 steps of history in front; steps before the
 //               sequence start are zero-filled by TMA, which is the conv's causal padding) and [n_out x 64] boxes
 //               of W_x (128-byte swizzle), each in a small ring.
@@ -44,6 +44,10 @@ constexpr int MMA_M = 128;
 #ifndef HX_CX_WS
 #define HX_CX_WS 2
 #endif
+// CTAs per SM up to which a tile is shared by the CTAs of a cluster
+#ifndef HX_CX_SPLIT_CTAS
+#define HX_CX_SPLIT_CTAS 2
+#endif
 #ifndef HX_CX_AB
 #define HX_CX_AB 2
 #endif
@@ -63,6 +67,9 @@ template <int TM> struct Cfg {
     static constexpr int X_STAGE_BYTES = (X_BOX_BYTES + 127) / 128 * 128;
     static constexpr int ROWS_PER_THREAD = TM / (COMPUTE_THREADS / 32);
     static constexpr int CTAS_PER_SM = TM == 64 ? 3 : 2;
+    // the partial tile of a split CTA ([TM] rows of part_stride floats) lies over the W_x and x rings
+    static_assert(TM != 64 || 64 * (256 + 4) * 4 <= WS * 256 * KC * 2 + XS * X_STAGE_BYTES, "partial tile does not fit (n_out 256)");
+    static_assert(TM != 64 || 64 * (16 + 4) * 4 <= WS * 16 * KC * 2 + XS * X_STAGE_BYTES, "partial tile does not fit (n_out 16)");
 };
 
 __host__ __device__ constexpr int w_stage_bytes(int n_out) { return (n_out * KC * 2 + 1023) / 1024 * 1024; }
@@ -93,12 +100,27 @@ __device__ __forceinline__ bool compute_sync_or(bool v) {
     return r != 0;
 }
 
-template <int TM>
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes of the shared memory of the cluster's CTA `rank`, at this CTA's address `addr`
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+// Row stride (floats) of the partial x_dbl tile a CTA of a cluster leaves in shared memory: 4 more than n_mma (a multiple of
+// 16), so that the 16-byte stores of eight neighbouring rows fall into different banks.
+__host__ __device__ constexpr int part_stride(int n_mma) { return n_mma + 4; }
+
+template <int TM, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, Cfg<TM>::CTAS_PER_SM)
 conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_u, const float *__restrict__ cw, const float *__restrict__ cb,
                   __nv_bfloat16 *__restrict__ xd, int64_t ldxd, int L, int E, int n_out, int n_mma, int tiles_per_seq,
-                  uint32_t tmem_cols) {
+                  uint32_t tmem_cols, int split) {
     constexpr int A_BYTES = Cfg<TM>::A_BYTES, X_BOX_BYTES = Cfg<TM>::X_BOX_BYTES, X_STAGE_BYTES = Cfg<TM>::X_STAGE_BYTES;
     constexpr int ROWS_PER_THREAD = Cfg<TM>::ROWS_PER_THREAD;
     extern __shared__ __align__(16) char smem_raw[];
@@ -120,9 +142,12 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     const uint32_t bar_acc_full = bar0 + 8u * (2 * XS + 2 * WS + 2 * AB);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x / tiles_per_seq;
-    const int t0 = (blockIdx.x % tiles_per_seq) * TM;
-    const int kblocks = E / KC;
+    // SPLIT: the `split` CTAs of a cluster share the tile, each walks its own run of the channel blocks
+    const int tile = SPLIT ? blockIdx.x / split : blockIdx.x, rank = SPLIT ? blockIdx.x % split : 0;
+    const int b = tile / tiles_per_seq;
+    const int t0 = (tile % tiles_per_seq) * TM;
+    const int kb0 = SPLIT ? rank * (E / KC) / split : 0;                          // first channel block
+    const int kblocks = SPLIT ? (rank + 1) * (E / KC) / split - kb0 : E / KC;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NBARS; ++i) mbar_init(bar0 + 8u * i, 1);
@@ -148,7 +173,7 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 const int sx = kb % XS;
                 if (!wait_or_abort(bar_x_empty(sx), ((kb / XS) & 1) ^ 1, abort_flag)) break;
                 mbar_expect_tx(bar_x_full(sx), X_BOX_BYTES);
-                tma_load_3d(smem_u32(x_tile + sx * X_STAGE_BYTES), &tm_x, bar_x_full(sx), kb * KC, t0 - HALO, b);
+                tma_load_3d(smem_u32(x_tile + sx * X_STAGE_BYTES), &tm_x, bar_x_full(sx), (kb0 + kb) * KC, t0 - HALO, b);
             }
         } else if (lane == 1) {
             tma_prefetch_desc(&tm_w);
@@ -156,7 +181,7 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 const int sw = kb % WS;
                 if (!wait_or_abort(bar_w_empty(sw), ((kb / WS) & 1) ^ 1, abort_flag)) break;
                 mbar_expect_tx(bar_w_full(sw), (uint32_t)(n_mma * KC * 2));
-                tma_load_2d(smem_u32(w_tile + sw * wbytes), &tm_w, bar_w_full(sw), kb * KC, 0);
+                tma_load_2d(smem_u32(w_tile + sw * wbytes), &tm_w, bar_w_full(sw), (kb0 + kb) * KC, 0);
             }
         }
     } else if (warp == 1) {
@@ -187,14 +212,15 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         const float4 *cw4 = reinterpret_cast<const float4 *>(cw);
         bool bad = false;
         // this block's taps and bias; the next block's are fetched while this one is computed
-        float4 wa_n = __ldg(cw4 + 2 * cp), wb_n = __ldg(cw4 + 2 * cp + 1);
-        float ba_n = cb ? __ldg(cb + 2 * cp) : 0.f, bb_n = cb ? __ldg(cb + 2 * cp + 1) : 0.f;
+        const int c0 = kb0 * KC + 2 * cp;
+        float4 wa_n = __ldg(cw4 + c0), wb_n = __ldg(cw4 + c0 + 1);
+        float ba_n = cb ? __ldg(cb + c0) : 0.f, bb_n = cb ? __ldg(cb + c0 + 1) : 0.f;
         for (int kb = 0; kb < kblocks; ++kb) {
             const int sx = kb % XS, ab = kb % AB;
             const float4 wa = wa_n, wb = wb_n;
             const float ba = ba_n, bb = bb_n;
             if (kb + 1 < kblocks) {
-                const int cn = (kb + 1) * KC + 2 * cp;
+                const int cn = (kb0 + kb + 1) * KC + 2 * cp;
                 wa_n = __ldg(cw4 + cn); wb_n = __ldg(cw4 + cn + 1);
                 if (cb) { ba_n = __ldg(cb + cn); bb_n = __ldg(cb + cn + 1); }
             }
@@ -230,7 +256,7 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
             bad = compute_sync_or(!ok || *abort_flag != 0);
             if (bad) break;
             if (ct == 0) {
-                tma_store_3d(&tm_u, smem_u32(a_tile + ab * A_BYTES), kb * KC, t0, b);
+                tma_store_3d(&tm_u, smem_u32(a_tile + ab * A_BYTES), (kb0 + kb) * KC, t0, b);
                 tma_store_commit();
                 mbar_arrive(bar_a_full(ab));
                 mbar_arrive(bar_x_empty(sx));
@@ -243,6 +269,8 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 tc_fence_after();
                 const int t = t0 + wq * 32 + lane;
                 __nv_bfloat16 *row = xd + ((int64_t)b * L + t) * ldxd;
+                // (SPLIT) this CTA's fp32 partial sums, over the rings of W_x and x: every box of theirs has been used
+                float *part = reinterpret_cast<float *>(w_tile) + (wq * 32 + lane) * part_stride(n_mma);
                 for (int c0 = 0; c0 < n_mma; c0 += 32) {
                     const uint32_t taddr = tmem_base + c0 + ((uint32_t)(wq * 32) << 16);
                     uint32_t r[32];
@@ -256,7 +284,14 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 #pragma unroll
                         for (int j = 0; j < 16; ++j) { r[j] = h[j]; r[16 + j] = 0u; }
                     }
-                    if (t < L) {
+                    if constexpr (SPLIT) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (c0 + q * 4 < n_mma)
+                                *reinterpret_cast<float4 *>(part + c0 + q * 4) =
+                                    make_float4(__uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]),
+                                                __uint_as_float(r[q * 4 + 2]), __uint_as_float(r[q * 4 + 3]));
+                    } else if (t < L) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             if (c0 + q * 8 < n_out) {   // n_out is a multiple of 8: whole 16-byte groups
@@ -275,6 +310,36 @@ conv_xproj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
             }
         }
         if (ct == 0) tma_store_wait_all<0>();  // the u tiles must outlive their TMA stores
+    }
+
+    if constexpr (SPLIT) {
+        // x_dbl = the sum of the cluster's partial tiles in rank order; every CTA adds and writes its share of the
+        // 8-column groups.  The second barrier keeps a CTA's shared memory alive until its peers have read it.
+        __syncthreads();
+        cluster_sync_all();
+        const uint32_t part0 = smem_u32(w_tile);
+        const int groups = n_out / 8;
+        for (int i = rank * THREADS + threadIdx.x; i < TM * groups; i += split * THREADS) {
+            const int r = i / groups, c = (i % groups) * 8;
+            const uint32_t at = part0 + (uint32_t)(r * part_stride(n_mma) + c) * 4;
+            float v[8] = {};
+            for (int k = 0; k < split; ++k) {
+                const float4 p0 = ld_cluster4(at, k), p1 = ld_cluster4(at + 16, k);
+                v[0] += p0.x; v[1] += p0.y; v[2] += p0.z; v[3] += p0.w;
+                v[4] += p1.x; v[5] += p1.y; v[6] += p1.z; v[7] += p1.w;
+            }
+            if (t0 + r < L) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+                    w[e] = *reinterpret_cast<const uint32_t *>(&h2);
+                }
+                *reinterpret_cast<uint4 *>(xd + ((int64_t)b * L + t0 + r) * ldxd + c) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+        __syncthreads();
+        cluster_sync_all();
     }
 
     // teardown: everybody meets, then the allocating warp frees tensor memory
@@ -302,10 +367,10 @@ hx_status read_status_convx(int *v, bool clear) {
 namespace hx {
 namespace cx {
 
-template <int TM>
+template <int TM, bool SPLIT>
 static hx_status launch(const void *x, int64_t x_batch_stride, int64_t x_row_stride, const float *conv_w, const float *conv_b,
                         const void *W_x, int64_t ldw, void *u, int64_t u_batch_stride, int64_t u_row_stride, void *x_dbl,
-                        int64_t x_dbl_row_stride, int batch, int seq_len, int d_inner, int n_out, cudaStream_t st) {
+                        int64_t x_dbl_row_stride, int batch, int seq_len, int d_inner, int n_out, int split, cudaStream_t st) {
     CUtensorMap mx, mw, mu;
     hx_status s;
     const uint64_t dims_x[3] = {(uint64_t)d_inner, (uint64_t)seq_len, (uint64_t)batch};
@@ -325,15 +390,26 @@ static hx_status launch(const void *x, int64_t x_batch_stride, int64_t x_row_str
     int dev = 0;
     HX_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && attr_set[dev].load(std::memory_order_acquire) < smem) {
-        HX_CUDA(cudaFuncSetAttribute(conv_xproj_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HX_CUDA(cudaFuncSetAttribute(conv_xproj_kernel<TM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev].store(smem, std::memory_order_release);
     }
     uint32_t cols = 32;
     while ((int)cols < n_mma) cols *= 2;
     const int tiles_per_seq = (seq_len + TM - 1) / TM;
-    conv_xproj_kernel<TM><<<batch * tiles_per_seq, THREADS, smem, st>>>(mx, mw, mu, conv_w, conv_b, static_cast<__nv_bfloat16 *>(x_dbl),
-                                                                       x_dbl_row_stride, seq_len, d_inner, n_out, n_mma,
-                                                                       tiles_per_seq, cols);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(batch * tiles_per_seq * split));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = split;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = SPLIT ? 1 : 0;
+    HX_CUDA(cudaLaunchKernelEx(&cfg, conv_xproj_kernel<TM, SPLIT>, mx, mw, mu, conv_w, conv_b, static_cast<__nv_bfloat16 *>(x_dbl),
+                               x_dbl_row_stride, seq_len, d_inner, n_out, n_mma, tiles_per_seq, cols, split));
     return check_launch("conv_xproj_kernel");
 }
 
@@ -362,9 +438,18 @@ extern "C" hx_status hx_conv1d_silu_xproj_fwd(const void *x, int64_t x_batch_str
     // one block after the other, so a short grid is bound by that chain: 33.7 against 25.5 us at 4 x 2048 x 1536)
     const int64_t long_tiles = (int64_t)batch * ((seq_len + 127) / 128);
     cudaStream_t st = (cudaStream_t)stream;
-    if (long_tiles < hx::sm_count())
-        return launch<64>(x, x_batch_stride, x_row_stride, conv_w, conv_b, W_x, ldw, u, u_batch_stride, u_row_stride, x_dbl,
-                          x_dbl_row_stride, batch, seq_len, d_inner, n_out, st);
-    return launch<128>(x, x_batch_stride, x_row_stride, conv_w, conv_b, W_x, ldw, u, u_batch_stride, u_row_stride, x_dbl,
-                       x_dbl_row_stride, batch, seq_len, d_inner, n_out, st);
+    if (long_tiles >= hx::sm_count())
+        return launch<128, false>(x, x_batch_stride, x_row_stride, conv_w, conv_b, W_x, ldw, u, u_batch_stride, u_row_stride,
+                                  x_dbl, x_dbl_row_stride, batch, seq_len, d_inner, n_out, 1, st);
+    // Few tiles: a cluster of 2, 4 or 8 CTAs shares one, each walking its part of the channels (the chain above), and adds
+    // its partial x_dbl through distributed shared memory, as long as the CTAs still find two places an SM: 23.1 -> 9.9 us
+    // for prompts of 60 to 731 steps (1 to 12 tiles), 23.8 -> 20.4 at 4 x 2048 (128 tiles, two CTAs each).
+    const int64_t tiles = (int64_t)batch * ((seq_len + 63) / 64);
+    int split = 1;
+    while (split < 8 && 2 * split <= d_inner / KC && tiles * 2 * split <= HX_CX_SPLIT_CTAS * (int64_t)hx::sm_count()) split *= 2;
+    if (split > 1)
+        return launch<64, true>(x, x_batch_stride, x_row_stride, conv_w, conv_b, W_x, ldw, u, u_batch_stride, u_row_stride, x_dbl,
+                                x_dbl_row_stride, batch, seq_len, d_inner, n_out, split, st);
+    return launch<64, false>(x, x_batch_stride, x_row_stride, conv_w, conv_b, W_x, ldw, u, u_batch_stride, u_row_stride, x_dbl,
+                             x_dbl_row_stride, batch, seq_len, d_inner, n_out, 1, st);
 }

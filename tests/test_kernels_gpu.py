@@ -118,6 +118,12 @@ def test_conv_silu_and_x_proj_in_one_kernel(B, L, E, NO):
     assert torch.equal(u2, ops.conv1d_silu(x_d, to_dev(cw), None))
 
 
+@pytest.mark.parametrize("B,L,E,NO", [(1, 40, 1536, 80), (1, 200, 576, 24), (2, 64, 512, 256), (5, 65, 448, 8), (4, 2048, 128, 80)])
+def test_conv_silu_and_x_proj_shared_tiles(B, L, E, NO):
+    """Few tiles: 2, 4 or 8 CTAs share one (576 and 448 channels: nine and seven blocks, unevenly)."""
+    test_conv_silu_and_x_proj_in_one_kernel(B, L, E, NO)
+
+
 def test_conv_silu_and_x_proj_rejects_what_it_does_not_take():
     import torch
     from helixml_b200 import _lib, ops
