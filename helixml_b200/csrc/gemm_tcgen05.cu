@@ -86,12 +86,12 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {
 }
 
 template <int BN, int PAIR = 0> struct TcCfg {
-    static constexpr int STAGES = PAIR ? 6 : (BN == 256 ? 4 : 6);
+    static constexpr int STAGES = PAIR ? 6 : (BN == 256 ? 4 : BN == 192 ? 4 : BN == 128 ? 6 : 8);
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_ROWS = PAIR ? BN / 2 : BN;   // W rows this CTA loads per stage
     static constexpr int B_BYTES = B_ROWS * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int TMEM_COLS = 2 * BN;
+    static constexpr int TMEM_COLS = BN == 192 ? 512 : 2 * BN;   // two accumulators; an allocation is a power of two
     static constexpr int OUT_STAGE_BYTES = 32 * 128;  // one epilogue warp's [32 rows x 128 bytes] staging tile
     static constexpr int OUT_BUFS = 2;                // staging tiles per epilogue warp (more of them change nothing)
     static constexpr int OUT_BYTES = 4 * OUT_BUFS * OUT_STAGE_BYTES;
@@ -467,6 +467,24 @@ static hx_status launch_tc_epi(const CUtensorMap &ma, const CUtensorMap &mw, con
     }
 }
 
+// Columns of a tile.  A CTA pulls (128 + BN) * 128 bytes of operands per k-block, which is also about what its tile costs
+// in time (0.15 us + 0.0011 us per column and k-block, alone on an SM or with every SM at work), so the plan is the one with
+// the smallest waves * (128 + BN); a narrower tile has to win by 4 % (it reads more operand bytes in all).
+// Against 256 columns everywhere: out_proj (K = 1536, 768 columns) 15.5 -> 11.4 us at up to 731 rows (64 columns), 27.3 -> 24.5
+// at 8192 rows (192); in_proj (K = 768, 3072 columns) 11.0 -> 8.0 to 8.9 (64 or 128 columns) at up to 731 rows.
+static int tile_columns(int M, int N) {
+    const int64_t m_tiles = (M + BM - 1) / BM, sms = sm_count();
+    int best = 0;
+    double best_cost = 0.;
+    for (int bn = 256; bn >= 64; bn -= 64) {
+        if (bn > 64 && bn - 64 >= N) continue;   // a whole 64-column group of zeros
+        const int64_t tiles = m_tiles * ((N + bn - 1) / bn);
+        const double cost = (double)((tiles + sms - 1) / sms) * (128 + bn);
+        if (best == 0 || cost < 0.96 * best_cost) { best = bn; best_cost = cost; }
+    }
+    return best;
+}
+
 }  // namespace gemm
 
 hx_status read_status_gemm(int *v, bool clear) {
@@ -521,7 +539,7 @@ extern "C" hx_status hx_gemm_bf16_cols(const void *A, int64_t lda, const void *W
     if (K <= 64 && M > 64 && N % 8 == 0 && N >= 64 && c_dtype == HX_BF16 && bias == nullptr && epilogue == kEpiNone &&
         (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc * 2) % 16 == 0)
         return launch_lowk(A, lda, W, ldw, C, ldc, M, N, K, st);
-    const int BN = N > 128 ? 256 : 128;
+    const int BN = tile_columns(M, N);
     CUtensorMap ma, mw;
     const uint64_t dims_a[2] = {(uint64_t)K, (uint64_t)M}, dims_w[2] = {(uint64_t)K, (uint64_t)N};
     const uint64_t str_a[1] = {(uint64_t)lda * 2}, str_w[1] = {(uint64_t)ldw * 2};
@@ -546,15 +564,15 @@ extern "C" hx_status hx_gemm_bf16_cols(const void *A, int64_t lda, const void *W
     // Mode 1 therefore takes pairs for the accumulating epilogue on at least four waves of them, mode 2 wherever the
     // shape allows.
     const int pm = pair_mode();
-    if (BN == 256 && vec_ok && pm != 0 && M >= 4 * BM && (epilogue == kEpiNone || (epilogue == kEpiAccumulate && c_dtype == HX_F32))) {
+    if (N > 128 && vec_ok && pm != 0 && M >= 4 * BM && (epilogue == kEpiNone || (epilogue == kEpiAccumulate && c_dtype == HX_F32))) {
         const bool accum = epilogue == kEpiAccumulate;
-        const int64_t pair_tiles = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+        const int64_t pair_tiles = (int64_t)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
         int pairs = 0;
         if (accum) pairs = pair_capacity<256, float, kEpiAccumulate>();
         else if (pm >= 2) pairs = c_dtype == HX_BF16 ? pair_capacity<256, __nv_bfloat16, kEpiNone>() : pair_capacity<256, float, kEpiNone>();
         if (pairs > 0 && (pm >= 2 || pair_tiles >= 4 * (int64_t)pairs)) {
             CUtensorMap mwh;
-            const uint32_t box_wh[2] = {(uint32_t)BK, (uint32_t)(BN / 2)};
+            const uint32_t box_wh[2] = {(uint32_t)BK, 128u};
             if ((s = hx::encode_tensor_map(&mwh, HX_BF16, 2, W, dims_w, str_w, box_wh, true)) != HX_OK) return s;
             if (accum) return launch_tc_pair_inst<256, float, kEpiAccumulate>(ma, mwh, mc, bias, C, ldc, M, N, K, epi_col0, pairs, st);
             if (c_dtype == HX_BF16)
@@ -562,10 +580,15 @@ extern "C" hx_status hx_gemm_bf16_cols(const void *A, int64_t lda, const void *W
             return launch_tc_pair_inst<256, float, kEpiNone>(ma, mwh, mc, bias, C, ldc, M, N, K, epi_col0, pairs, st);
         }
     }
-    if (BN == 256) {
-        if (c_dtype == HX_BF16) return launch_tc_epi<256, __nv_bfloat16>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st);
-        return launch_tc_epi<256, float>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st);
+#define HX_TC_TILE(COLS)                                                                                                          \
+    return c_dtype == HX_BF16                                                                                                     \
+               ? launch_tc_epi<COLS, __nv_bfloat16>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st)              \
+               : launch_tc_epi<COLS, float>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st)
+    switch (BN) {
+        case 64: HX_TC_TILE(64);
+        case 128: HX_TC_TILE(128);
+        case 192: HX_TC_TILE(192);
+        default: HX_TC_TILE(256);
     }
-    if (c_dtype == HX_BF16) return launch_tc_epi<128, __nv_bfloat16>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st);
-    return launch_tc_epi<128, float>(ma, mw, mc, bias, C, ldc, M, N, K, vec_ok, epilogue, epi_col0, st);
+#undef HX_TC_TILE
 }

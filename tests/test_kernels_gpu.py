@@ -178,6 +178,29 @@ def test_gemm_simt_f32(M, N, K):
     assert fp32_tol_err(to_np(got), cbind.linear(a, w, b)) <= FP32_TOL
 
 
+@pytest.mark.parametrize("M,N,K", [(100, 768, 136), (129, 72, 200), (2000, 768, 72), (2050, 776, 136), (4096, 768, 72), (4100, 584, 136),
+                                   (10000, 1000, 72)])
+def test_gemm_tcgen05_tile_widths(M, N, K):
+    """Tiles of 64, 128, 192 and 256 columns (by M and N), ragged in both directions: plain, accumulating and activated
+    results, and a C that the TMA store does not take."""
+    import torch
+    from helixml_b200 import _lib, ops
+    a = synth.round_bf16(synth.normal(64, "a", (M, K)))
+    w = synth.round_bf16(synth.normal(64, "w", (N, K), 0, 0.05))
+    a_d, w_d = to_dev(a, "bf16"), to_dev(w, "bf16")
+    ref = a.astype(np.float64) @ w.astype(np.float64).T
+    assert rel_l2(to_np(ops.gemm(a_d, w_d)), ref) <= 5e-3
+    c = torch.ones(M, N, device="cuda")
+    ops.gemm_acc(a_d, w_d, c)
+    assert fp32_tol_err(to_np(c), ref + 1.0) <= FP32_TOL
+    got = ops.gemm(a_d, w_d, out_dtype=torch.float32, epilogue=_lib.EPI_SILU)
+    assert fp32_tol_err(to_np(got), ref / (1.0 + np.exp(-ref))) <= FP32_TOL
+    odd = torch.full((M, N + 1), 7.0, device="cuda")
+    ops.gemm(a_d, w_d, out_dtype=torch.float32, out=odd[:, :N])
+    assert fp32_tol_err(to_np(odd[:, :N]), ref) <= FP32_TOL and bool((odd[:, N] == 7.0).all())
+    _status_ok()
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("M,N,K", [(31, 33, 61), (33, 31, 64), (32, 32, 130), (700, 641, 35), (641, 700, 36), (1500, 1400, 9),
                                    (1409, 1536, 24)])
