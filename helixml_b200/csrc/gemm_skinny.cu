@@ -10,7 +10,8 @@
 // long as A and B agree, so inside a block of 32 k values lane (g, tid) loads the 8 consecutive elements
 // k = 8 tid .. 8 tid + 7 of its row and uses them as the two k-halves of two MMAs:
 //   MMA j (j = 0, 1): "k pair 2 tid" = elements 4 j + {0, 1}, "k pair 2 tid + 8" = elements 4 j + {2, 3}.
-// A comes straight from global memory (it is M x K, a few tens of KB, shared by every CTA through L2/L1).
+// A comes straight from global memory (it is M x K, a few tens of KB, shared by every CTA through L2/L1).  A, C and the bias
+// carry no __restrict__: their loads must stay behind chain_wait().
 #include "gemm.cuh"
 
 namespace hx {
@@ -20,8 +21,9 @@ constexpr int kSkinnyWarps = 16;
 
 template <int MT, typename TC, int EPI>
 __global__ void __launch_bounds__(kSkinnyWarps * 32)
-gemm_skinny_kernel(const __nv_bfloat16 *__restrict__ A, int64_t lda, const __nv_bfloat16 *__restrict__ W, int64_t ldw,
-                   const float *__restrict__ bias, TC *__restrict__ C, int64_t ldc, int M, int N, int K, int epi_col0) {
+gemm_skinny_kernel(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *__restrict__ W, int64_t ldw,
+                   const float *bias, TC *C, int64_t ldc, int M, int N, int K, int epi_col0) {
+    chain_trigger();
     __shared__ float partial[kSkinnyWarps * MT * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tid = lane & 3;
@@ -46,34 +48,50 @@ gemm_skinny_kernel(const __nv_bfloat16 *__restrict__ A, int64_t lda, const __nv_
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[mt][i] = 0.f;
 
-    // this warp's k-blocks: warp, warp + 16, ... ; two blocks per trip so that their loads overlap
-    for (int k0 = warp * 32; k0 < K; k0 += kSkinnyWarps * 64) {
-        uint4 b[2], a[2][MT][2];
+    // this warp's k-blocks: warp, warp + 16, ...  Four blocks of W per trip (inner dimensions up to 2048 in one), A two
+    // blocks at a time.  W does not depend on the kernel before this one, so the first trip's are requested before waiting.
+    uint4 b[4];
+    auto fetch_w = [&](int k0) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < 4; ++u) {
             const int k = k0 + u * kSkinnyWarps * 32;
-            const bool k_ok = k < K;
-            b[u] = (n_ok && k_ok) ? *reinterpret_cast<const uint4 *>(wrow + k) : zero4;
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    a[u][mt][h] = (a_ok[mt][h] && k_ok) ? *reinterpret_cast<const uint4 *>(arow[mt][h] + k) : zero4;
+            b[u] = (n_ok && k < K) ? *reinterpret_cast<const uint4 *>(wrow + k) : zero4;
         }
+    };
+    fetch_w(warp * 32);
+    chain_wait();
+    for (int k0 = warp * 32; k0 < K; k0 += kSkinnyWarps * 128) {
+        if (k0 != warp * 32) fetch_w(k0);
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int half = 0; half < 2; ++half) {
+            if (k0 + half * kSkinnyWarps * 64 >= K) break;   // warp-uniform
+            uint4 a[2][MT][2];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                // fragment registers: a0 = (row g, k pair), a1 = (row g+8, k pair), a2 = (row g, k pair + 8), a3 = (row g+8, ...)
-                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                             "{%0, %1, %2, %3};"
-                             : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
-                             : "r"(a[u][mt][0].x), "r"(a[u][mt][1].x), "r"(a[u][mt][0].y), "r"(a[u][mt][1].y), "r"(b[u].x), "r"(b[u].y));
-                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                             "{%0, %1, %2, %3};"
-                             : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
-                             : "r"(a[u][mt][0].z), "r"(a[u][mt][1].z), "r"(a[u][mt][0].w), "r"(a[u][mt][1].w), "r"(b[u].z), "r"(b[u].w));
+            for (int u = 0; u < 2; ++u) {
+                const int k = k0 + (half * 2 + u) * kSkinnyWarps * 32;
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        a[u][mt][h] = (a_ok[mt][h] && k < K) ? *reinterpret_cast<const uint4 *>(arow[mt][h] + k) : zero4;
             }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint4 bu = b[half * 2 + u];
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    // fragment registers: a0 = (row g, k pair), a1 = (row g+8, k pair), a2 = (row g, k pair + 8), a3 = (row g+8, ...)
+                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                                 "{%0, %1, %2, %3};"
+                                 : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                                 : "r"(a[u][mt][0].x), "r"(a[u][mt][1].x), "r"(a[u][mt][0].y), "r"(a[u][mt][1].y), "r"(bu.x), "r"(bu.y));
+                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                                 "{%0, %1, %2, %3};"
+                                 : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                                 : "r"(a[u][mt][0].z), "r"(a[u][mt][1].z), "r"(a[u][mt][0].w), "r"(a[u][mt][1].w), "r"(bu.z), "r"(bu.w));
+                }
+            }
+        }
     }
     // partial[warp][mt][lane][i]; accumulator layout: i = 0, 1 -> (row g, columns 2 tid, 2 tid + 1); i = 2, 3 -> row g + 8
 #pragma unroll
@@ -98,30 +116,32 @@ gemm_skinny_kernel(const __nv_bfloat16 *__restrict__ A, int64_t lda, const __nv_
 
 template <int MT, typename TC>
 static hx_status launch_skinny_epi(const void *A, int64_t lda, const void *W, int64_t ldw, const float *bias, void *C, int64_t ldc,
-                                   int M, int N, int K, int epi, int epi_col0, cudaStream_t st) {
+                                   int M, int N, int K, int epi, int epi_col0, cudaStream_t st, bool chain) {
     const dim3 grid((unsigned)((N + 7) / 8)), block(kSkinnyWarps * 32);
     auto a = static_cast<const __nv_bfloat16 *>(A), w = static_cast<const __nv_bfloat16 *>(W);
     auto c = static_cast<TC *>(C);
+    cudaError_t e = cudaSuccess;
     switch (epi) {
-        case kEpiNone: gemm_skinny_kernel<MT, TC, kEpiNone><<<grid, block, 0, st>>>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSilu: gemm_skinny_kernel<MT, TC, kEpiSilu><<<grid, block, 0, st>>>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSoftplus: gemm_skinny_kernel<MT, TC, kEpiSoftplus><<<grid, block, 0, st>>>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSiluFast: gemm_skinny_kernel<MT, TC, kEpiSiluFast><<<grid, block, 0, st>>>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
+        case kEpiNone: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiNone>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
+        case kEpiSilu: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSilu>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
+        case kEpiSoftplus: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSoftplus>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
+        case kEpiSiluFast: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSiluFast>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
         case kEpiAccumulate:
-            if constexpr (sizeof(TC) == 4) gemm_skinny_kernel<MT, TC, kEpiAccumulate><<<grid, block, 0, st>>>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0);
+            if constexpr (sizeof(TC) == 4) e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiAccumulate>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0);
             else return fail(HX_ERR_DTYPE_MISMATCH, "accumulating GEMM needs an fp32 C");
             break;
         default: return fail(HX_ERR_INVALID_INPUT, "unknown epilogue %d", epi);
     }
+    HX_CUDA(e);
     return check_launch("gemm_skinny_kernel");
 }
 
 // M <= 64, K a multiple of 32, lda / ldw multiples of 8 and 16-byte aligned bases (checked by the caller).
 hx_status launch_skinny(const void *A, int64_t lda, const void *W, int64_t ldw, const float *bias, void *C, int64_t ldc,
-                        int c_dtype, int M, int N, int K, int epi, int epi_col0, cudaStream_t st) {
+                        int c_dtype, int M, int N, int K, int epi, int epi_col0, cudaStream_t st, bool chain) {
 #define HX_SKINNY(MT)                                                                                                   \
-    return c_dtype == HX_BF16 ? launch_skinny_epi<MT, __nv_bfloat16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, epi_col0, st)    \
-                              : launch_skinny_epi<MT, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, epi_col0, st)
+    return c_dtype == HX_BF16 ? launch_skinny_epi<MT, __nv_bfloat16>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, epi_col0, st, chain)    \
+                              : launch_skinny_epi<MT, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, epi_col0, st, chain)
     if (M <= 16) { HX_SKINNY(1); }
     if (M <= 32) { HX_SKINNY(2); }
     HX_SKINNY(4);

@@ -529,12 +529,12 @@ size_t MambaBlock::step_workspace_bytes(int64_t batch) const {
 }
 
 Result<Unit> MambaBlock::step_into(const void *x, void *out, int64_t batch, float *h, void *conv_state, void *workspace,
-                                   size_t ws_bytes, void *stream, float *residual, const float *norm_w, float norm_eps) const {
+                                   size_t ws_bytes, void *stream, float *residual, const float *norm_w, float norm_eps, bool chained) const {
     hx_mamba_step_args a = step_args(*this, batch);
     a.x = x; a.out = out; a.h = h; a.conv_state = conv_state;
     a.workspace = workspace; a.workspace_bytes = ws_bytes;
     a.residual = residual; a.norm_w = norm_w; a.norm_eps = norm_eps;
-    HELIX_TRY_ABI(hx_mamba_block_step(&a, stream));
+    HELIX_TRY_ABI(hx::mamba_block_step(&a, chained, stream));
     return Unit{};
 }
 
@@ -851,7 +851,7 @@ Result<Unit> ByteLM::enqueue_step(void *stream) {
         // output is added into the stream by out_proj
         HELIX_TRY(blocks[l]->step_into(nullptr, dec_->block_out.data(), B, static_cast<float *>(dec_->h[l].data()),
                                        dec_->conv[l].data(), dec_->workspace.data(), (size_t)dec_->workspace.numel(), stream,
-                                       resid, static_cast<const float *>(norms[l]->weight.data()), eps));
+                                       resid, static_cast<const float *>(norms[l]->weight.data()), eps, true));
     }
     HELIX_TRY_ABI(hx_rmsnorm_fwd(nullptr, (int)dtype, resid, static_cast<const float *>(norm_f.data()),
                                  dec_->normed.data(), (int)dtype, B, (int)d_model, eps, stream));

@@ -217,7 +217,7 @@ class MambaBlock : public Module {
     // is added into residual (x may be NULL, out is scratch for the fp32 path).
     Result<Unit> step_into(const void *x, void *out, int64_t batch, float *h, void *conv_state, void *workspace,
                            size_t workspace_bytes, void *stream, float *residual = nullptr, const float *norm_w = nullptr,
-                           float norm_eps = 1e-5f) const;
+                           float norm_eps = 1e-5f, bool chained = false) const;
     // true when a residual-form step runs as four kernels (norm and conv step inside in_proj, add inside out_proj)
     bool step_is_fused(int64_t batch) const { return dtype == DType::BF16 && d_model % 32 == 0 && batch <= 64 && d_inner % 8 == 0; }
     size_t step_workspace_bytes(int64_t batch) const;

@@ -72,6 +72,48 @@ hx_status read_status_scan(int *v, bool clear);
 hx_status read_status_gemm(int *v, bool clear);
 hx_status read_status_convx(int *v, bool clear);
 
+// ---------------------------------------------------------------- chained launches
+// A decode step is about a hundred dependent kernels of a few microseconds.  Launched with `chain` set, a kernel starts
+// while its predecessor in the stream still runs, as soon as every CTA of that one has called chain_trigger(); before
+// chain_wait() returns it may touch nothing but constants (weights), and chain_wait() returns when the predecessor has
+// completed.  Every kernel of a chain therefore triggers first, fetches its weights, waits (in every thread) and goes on:
+// set-up and weight fetch of a kernel run under the one before it.  Launched without `chain`, both calls do nothing.
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... V>
+inline cudaError_t launch_chained_smem(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster,
+                                       cudaStream_t st, V... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (chain) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = 1;
+        at[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... V>
+inline cudaError_t launch_chained(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, V... args) {
+    return launch_chained_smem(chain, kernel, grid, block, 0, 1, st, args...);
+}
+
+// hx_mamba_block_step; `chained`: the kernel queued before this call on `stream` is part of the same decode step, so
+// nothing that writes a weight can still be running when the first kernel starts early (decode.cu).
+hx_status mamba_block_step(const hx_mamba_step_args *a, bool chained, void *stream);
+
 // ---------------------------------------------------------------- device-side helpers
 template <typename T> __device__ __forceinline__ float ld_f32(const T *p);
 template <> __device__ __forceinline__ float ld_f32<float>(const float *p) { return *p; }

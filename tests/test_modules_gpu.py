@@ -195,6 +195,38 @@ def test_byte_lm_prefill_then_decode_steps(dtype_name):
     assert np.array_equal(runs[0], runs[1])  # graph replay and plain launches agree bit for bit
 
 
+@pytest.mark.parametrize("B,M", [(1, 128), (16, 128), (17, 256), (32, 128), (33, 128), (64, 128), (65, 128), (3, 1152)])
+def test_byte_lm_decode_step_chain(B, M):
+    """The chained kernels of a step at the batch sizes where their tiles change (65: the unfused form) and at inner
+    dimensions past what is fetched ahead (1152): every step against the oracle, graph and plain launches bit for bit."""
+    import torch
+    from helixml_b200 import _lib, nn
+    nl, L0, steps = 2, 5, 4
+    emb, layers, normf = _lm_weights(11, nl, M)
+    layers = [{k: (synth.round_bf16(v) if k in ("W_in", "W_x", "W_dt", "W_out") else v) for k, v in l.items()} for l in layers]
+    emb = synth.round_bf16(emb)
+    tok = synth.random_bytes(11, "tok", (B, L0 + steps))
+    ref = cbind.byte_lm(tok, emb, layers, normf, 16, 4)[:, L0:]
+    tok_d = torch.from_numpy(tok).cuda()
+    runs = []
+    for graph in (True, False):
+        lm = nn.ByteLM(nl, M, dtype=nn.BF16)
+        lm.load_weights(emb, layers, normf)
+        lm.decode_graph(graph)
+        pre = torch.empty(B, L0, 256, device="cuda", dtype=torch.bfloat16)
+        got = torch.empty(steps, B, 256, device="cuda", dtype=torch.bfloat16)
+        first = tok_d[:, :L0].contiguous()
+        nxt = tok_d[:, L0:].t().contiguous()
+        lm.prefill_device(first.data_ptr(), pre.data_ptr(), B, L0)
+        for s in range(steps):
+            lm.decode_step_device(nxt[s].data_ptr(), got[s].data_ptr(), B)
+        torch.cuda.synchronize()
+        assert _lib.device_status() == 0
+        runs.append(got.float().cpu().numpy().transpose(1, 0, 2))
+        assert rel_l2(runs[-1], ref) <= BF16_TOL
+    assert np.array_equal(runs[0], runs[1])
+
+
 def test_byte_lm_decode_without_prefill_is_an_error():
     import torch
     from helixml_b200 import _lib, nn
