@@ -667,6 +667,10 @@ struct ByteLM::FwdGraphs {
     }
 };
 
+void ByteLM::drop_forwards() {
+    if (fwd_) fwd_->clear();
+}
+
 void ByteLM::set_forward_graph(bool enable) {
     std::lock_guard<std::recursive_mutex> lock(mu_);
     forward_graph_ = enable;
@@ -743,13 +747,13 @@ Result<Unit> ByteLM::parameters_updated() {
 
 // Makes the activation buffers hold (batch, seq_len).  They only ever grow, by at least half of what they are: prompts of
 // changing length run in the same memory (allocating per shape cost 1 to 100 ms a prompt, and every captured forward with
-// it, since cudaFree waits for the device).  `moved` tells that captured forwards point into memory that is gone.
-Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len, bool *moved) {
-    if (moved) *moved = false;
+// it, since cudaFree waits for the device).  Captured forwards point into these buffers and into the decode state, so
+// both functions drop them before they replace any of it: no caller has to.
+Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len) {
     const int64_t T = batch * seq_len;
     if (!buf_) buf_ = new Buffers();
     if (T > buf_->tokens_cap) {
-        if (moved) *moved = true;
+        drop_forwards();
         const int64_t grown = buf_->tokens_cap + buf_->tokens_cap / 2;
         const int64_t cap = T > grown ? T : grown;
         delete buf_;
@@ -777,7 +781,7 @@ Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len, bool *moved)
     }
     const size_t wb = blocks[0]->workspace_bytes(batch, seq_len);
     if (wb > buf_->workspace_cap) {
-        if (moved) *moved = true;
+        drop_forwards();
         const size_t cap = std::max(wb, buf_->workspace_cap + buf_->workspace_cap / 2);
         buf_->workspace_cap = 0;
         buf_->workspace = DeviceTensor();
@@ -811,14 +815,13 @@ Result<Unit> ByteLM::prefill_device(const uint8_t *tokens_dev, void *logits_dev,
     return run_layers(tokens_dev, logits_dev, batch, seq_len, stream, true);
 }
 
-// The decode state of `batch` sequences.  The buffers grow only; `moved` as for ensure_buffers.
-Result<Unit> ByteLM::ensure_decode(int64_t batch, bool *moved) {
-    if (moved) *moved = false;
+// The decode state of `batch` sequences.  The buffers grow only.
+Result<Unit> ByteLM::ensure_decode(int64_t batch) {
     if (dec_ && dec_->cap >= batch) {
         dec_->batch = batch;
         return Unit{};
     }
-    if (moved) *moved = true;
+    drop_forwards();
     delete dec_;
     dec_ = new Decode();
     const MambaBlock &b0 = *blocks[0];
@@ -922,18 +925,13 @@ Result<Unit> ByteLM::run_layers(const uint8_t *tokens_dev, void *logits_dev, int
     std::lock_guard<std::recursive_mutex> lock(mu_);
     if (batch <= 0 || seq_len <= 0) return err(HX_ERR_INVALID_DIMENSION, "ByteLM: batch and seq_len must be positive");
     HELIX_TRY(use_device(device_));
-    bool moved = false;
-    auto eb = ensure_buffers(batch, seq_len, &moved);
-    if (moved && fwd_) fwd_->clear();  // the graphs point into the old activation buffers
-    if (!eb.ok()) return eb.error();
+    HELIX_TRY(ensure_buffers(batch, seq_len));
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing((cudaStream_t)stream, &cap);
     if (!forward_graph_ || prof_ || cap != cudaStreamCaptureStatusNone)
         return run_layers_plain(tokens_dev, logits_dev, batch, seq_len, stream, keep_state);
     if (keep_state) {
-        auto ed = ensure_decode(batch, &moved);  // allocate outside any capture
-        if (moved && fwd_) fwd_->clear();  // graphs that keep the state point into the old state buffers
-        if (!ed.ok()) return ed.error();
+        HELIX_TRY(ensure_decode(batch));  // allocate outside any capture
         dec_->steps = 0;
     }
     if (!fwd_) fwd_ = new FwdGraphs();
@@ -988,9 +986,9 @@ Result<Unit> ByteLM::run_layers(const uint8_t *tokens_dev, void *logits_dev, int
 
 Result<Unit> ByteLM::run_layers_plain(const uint8_t *tokens_dev, void *logits_dev, int64_t batch, int64_t seq_len, void *stream,
                                       bool keep_state) {
-    HELIX_TRY(ensure_buffers(batch, seq_len, nullptr));
+    HELIX_TRY(ensure_buffers(batch, seq_len));
     if (keep_state) {
-        HELIX_TRY(ensure_decode(batch, nullptr));
+        HELIX_TRY(ensure_decode(batch));
         dec_->steps = 0;
     }
     const int64_t T = batch * seq_len;
@@ -1047,10 +1045,7 @@ Result<Unit> ByteLM::forward_host(const uint8_t *tokens_host, void *logits_host,
     if (!tokens_host || !logits_host) return err(HX_ERR_INVALID_INPUT, "ByteLM::forward_host: NULL buffer");
     HELIX_TRY(use_device(device_));
     if (batch <= 0 || seq_len <= 0) return err(HX_ERR_INVALID_DIMENSION, "ByteLM: batch and seq_len must be positive");
-    bool moved = false;
-    auto eb = ensure_buffers(batch, seq_len, &moved);
-    if (moved && fwd_) fwd_->clear();
-    if (!eb.ok()) return eb.error();
+    HELIX_TRY(ensure_buffers(batch, seq_len));
     const int64_t T = batch * seq_len;
     HELIX_TRY_ABI(hx_memcpy_h2d(buf_->tokens.data(), tokens_host, (size_t)T, stream));
     HELIX_TRY(forward_device(static_cast<const uint8_t *>(buf_->tokens.data()), buf_->logits.data(), batch, seq_len, stream));

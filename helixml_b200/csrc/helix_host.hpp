@@ -297,8 +297,9 @@ class ByteLM : public Module {
     float eps = 1e-5f;
 
   private:
-    Result<Unit> ensure_buffers(int64_t batch, int64_t seq_len, bool *moved);
-    Result<Unit> ensure_decode(int64_t batch, bool *moved);
+    Result<Unit> ensure_buffers(int64_t batch, int64_t seq_len);
+    Result<Unit> ensure_decode(int64_t batch);
+    void drop_forwards();
     Result<Unit> enqueue_step(void *stream);
     Result<Unit> run_layers(const uint8_t *tokens_dev, void *logits_dev, int64_t batch, int64_t seq_len, void *stream,
                             bool keep_state);

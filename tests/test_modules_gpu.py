@@ -440,7 +440,7 @@ def test_byte_lm_forward_graph_replay_equals_plain_launches(dtype_name):
             lm.forward_device(buf.data_ptr(), out.data_ptr(), B, L)
             torch.cuda.synchronize()
             assert torch.equal(out, want[i]), (rnd, i)
-        # another shape in between drops the graphs (they point into the old activation buffers)
+        # a smaller shape in between uses the same buffers and leaves the graphs
         small = torch.empty(1, 64, 256, device="cuda", dtype=td)
         lm.forward_device(toks[0][:1, :64].contiguous().data_ptr(), small.data_ptr(), 1, 64)
     # prefill with state through the graph, then a decode step: same as with plain launches
@@ -515,6 +515,45 @@ def test_byte_lm_changing_lengths_share_buffers(lengths):
         for i, (B, L) in enumerate(shapes):
             got = run(lm, B, L, i)
             assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), (rnd, i)
+
+
+def test_byte_lm_captured_prefill_after_a_larger_profiled_one():
+    """A captured prefill, then a prefill of more sequences (and fewer tokens) that runs as plain launches because a profile
+    is on and replaces the decode state, then the first prefill again: it and the steps that follow equal a fresh model's
+    bit for bit."""
+    import torch
+    from helixml_b200 import _lib, nn
+    emb, layers, normf = _lm_weights(23, 2, 128)
+
+    def fresh():
+        lm = nn.ByteLM(2, 128)
+        lm.load_weights(emb, layers, normf)
+        return lm
+
+    tok = torch.from_numpy(synth.random_bytes(23, "t", (2, 100))).cuda()
+    wide = torch.from_numpy(synth.random_bytes(23, "w", (4, 20))).cuda()
+    nxt = torch.from_numpy(synth.random_bytes(23, "n", (3, 2))).cuda()
+    out = torch.empty(2, 100, 256, device="cuda", dtype=torch.bfloat16)
+    wide_out = torch.empty(4, 20, 256, device="cuda", dtype=torch.bfloat16)
+
+    def steps(lm):
+        lg = torch.empty(3, 2, 256, device="cuda", dtype=torch.bfloat16)
+        lm.prefill_device(tok.data_ptr(), out.data_ptr(), 2, 100)
+        for i in range(3):
+            lm.decode_step_device(nxt[i].data_ptr(), lg[i].data_ptr(), 2)
+        torch.cuda.synchronize()
+        return out.clone(), lg
+
+    want = steps(fresh())
+    lm = fresh()
+    for _ in range(3):  # plain, captured, replayed
+        lm.prefill_device(tok.data_ptr(), out.data_ptr(), 2, 100)
+    _lib.check(_lib.lib().hx_byte_lm_profile(lm._h, 1))
+    lm.prefill_device(wide.data_ptr(), wide_out.data_ptr(), 4, 20)
+    _lib.check(_lib.lib().hx_byte_lm_profile(lm._h, 0))
+    for _ in range(3):
+        got = steps(lm)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
 def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
