@@ -761,7 +761,8 @@ static void seg_plan(const hx_scan_args *a, int chunk, int *n_seg, int *seg_len)
 }
 
 constexpr int kChunkBf16 = 32, kChunkF32 = 32;
-constexpr int kPlanChunk = 32;  // segment lengths are multiples of this (of the direct kernel's 16 steps in the look-back form)
+constexpr int kPlanChunk = 32;          // segment lengths are multiples of this in the chained forms
+constexpr int kPlanChunkLookBack = 16;  // and of this, the direct kernel's chunk, in the look-back form
 
 static int tiles_of(const hx_scan_args *a) {
     const int DT = a->io_dtype == HX_BF16 ? 64 : 32;
@@ -1001,7 +1002,7 @@ static thread_local int t_orphan_from = 0;
 static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t st, int form = 0) {
     HX_REQUIRE(a->d_state == 16, HX_ERR_UNSUPPORTED_OPERATION, "the direct scan needs d_state == 16 (got %d)", a->d_state);
     const bool bf = a->io_dtype == HX_BF16;
-    const int ES = bf ? 2 : 4, BOXC = 128 / ES, TC = 16;
+    const int ES = bf ? 2 : 4, BOXC = 128 / ES, TC = kPlanChunkLookBack;
     if (form == 1)
         HX_REQUIRE(lookback_ok(a), HX_ERR_UNSUPPORTED_OPERATION,
                    "the look-back scan takes raw z and, with a fused dt projection, the block's configuration");
@@ -1009,7 +1010,7 @@ static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t s
     const int DT = bf ? (cpl == 2 ? 256 : 128) : 128;  // channels per CTA (4 consumer warps)
     const int tiles = (a->d_inner + DT - 1) / DT;
     int n_seg = 1, seg_len = (a->seq_len + TC - 1) / TC * TC;
-    if (split) seg_plan(a, form == 1 ? TC : kPlanChunk, &n_seg, &seg_len);
+    if (split) seg_plan(a, form == 1 ? kPlanChunkLookBack : kPlanChunk, &n_seg, &seg_len);
     if (n_seg <= 1) form = 0;
 
     TiledParams p;
@@ -1254,9 +1255,8 @@ hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *a, size_t *bytes
     if (a->variant != HX_SCAN_SEQSPLIT && a->variant != HX_SCAN_LOOKBACK && a->seq_splits <= 1) return HX_OK;
     if (a->variant == HX_SCAN_SIMPLE) return HX_OK;
     int n_seg, seg_len;
-    // the finer plan has the most segments, so the size serves every form the variant may run
-    const bool may_look_back = a->variant == HX_SCAN_AUTO || a->variant == HX_SCAN_LOOKBACK;
-    hx::scan::seg_plan(a, may_look_back ? 16 : hx::scan::kPlanChunk, &n_seg, &seg_len);
+    // the look-back form's plan has the most segments, so its size serves every form, whichever variant asks
+    hx::scan::seg_plan(a, hx::scan::kPlanChunkLookBack, &n_seg, &seg_len);
     *bytes = hx::scan::workspace_bytes(a, n_seg);
     return HX_OK;
 }
@@ -1353,8 +1353,10 @@ hx_status hx_selective_scan_fwd_noalloc(const hx_scan_args *a, void *stream) {
     if (a->batch == 0 || a->seq_len == 0 || a->d_inner == 0) return HX_OK;
     hx_scan_args b = *a;
     b.variant = HX_SCAN_SEQSPLIT;
-    size_t need = 0;
-    if ((s = hx_selective_scan_workspace_bytes(&b, &need)) != HX_OK) return s;
+    // what the chained form below uses (hx_selective_scan_workspace_bytes also covers the look-back form's finer plan)
+    int n_seg, seg_len;
+    hx::scan::seg_plan(&b, hx::scan::kPlanChunk, &n_seg, &seg_len);
+    const size_t need = hx::scan::workspace_bytes(&b, n_seg);
     HX_REQUIRE(need <= (size_t)HX_SCAN_NOALLOC_SCRATCH_BYTES, HX_ERR_INVALID_INPUT,
                "hx_selective_scan_fwd_noalloc: this problem needs %zu bytes of carry scratch, the built-in array holds "
                "%zu; use fewer seq_splits, a smaller batch * d_inner, or hx_selective_scan_fwd with your own workspace",

@@ -64,7 +64,7 @@ def scan_workspace_bytes(batch, seq_len, d_inner, dtype, seq_splits=0) -> int:
     a = L.ScanArgs()
     a.batch, a.seq_len, a.d_inner, a.d_state = batch, seq_len, d_inner, 16
     a.io_dtype = L.HX_BF16 if dtype == torch.bfloat16 else L.HX_F32
-    a.variant = L.SCAN_LOOKBACK  # the largest of the split forms
+    a.variant = L.SCAN_SEQSPLIT
     a.seq_splits = seq_splits
     n = C.c_size_t(0)
     L.check(L.lib().hx_selective_scan_workspace_bytes(C.byref(a), C.byref(n)))

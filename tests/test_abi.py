@@ -105,6 +105,15 @@ def test_workspace_size_queries():
     a.variant, a.seq_splits = L.SCAN_SEQSPLIT, 4
     assert lib.hx_selective_scan_workspace_bytes(C.byref(a), C.byref(n)) == 0
     assert n.value >= 3 * 2 * 128 * 16 * 4
+    # one size serves every split form, whichever variant asked for it (700 steps in 16: 15 segments look back, 11 chained)
+    for seq_len, splits in ((700, 16), (200, 5), (33, 2), (4096, 7)):
+        a.seq_len, a.seq_splits = seq_len, splits
+        sizes = set()
+        for v in (L.SCAN_AUTO, L.SCAN_TILED, L.SCAN_SEQSPLIT, L.SCAN_DIRECT, L.SCAN_LOOKBACK):
+            a.variant = v
+            assert lib.hx_selective_scan_workspace_bytes(C.byref(a), C.byref(n)) == 0
+            sizes.add(n.value)
+        assert len(sizes) == 1, sizes
     assert lib.hx_s4_ref_workspace_bytes(100, 16) == 100 * 16 * 4
     st = L.MambaStepArgs()
     st.batch, st.d_model, st.d_inner, st.d_state, st.d_conv, st.dt_rank, st.io_dtype = 4, 64, 128, 16, 4, 4, L.HX_F32

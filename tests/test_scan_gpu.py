@@ -564,6 +564,18 @@ def test_auto_lookback_general_decay(dtype, L, splits, mixed):
         check(hg, hr, dtype)
 
 
+def test_workspace_sized_for_chained_segments_serves_auto():
+    """A workspace of the size asked with HX_SCAN_SEQSPLIT, given to HX_SCAN_AUTO, which looks back in finer segments."""
+    import torch
+    from helixml_b200 import ops
+    inp = synth.scan_inputs(66, 2, 700, 96, 16, 4, bf16=True)
+    dev = {k: to_dev(v, "bf16" if k in ("x", "dt", "z", "B", "C") else None) for k, v in inp.items()}
+    ws = torch.empty(ops.scan_workspace_bytes(2, 700, 96, torch.bfloat16, 16), dtype=torch.uint8, device="cuda")
+    y = ops.selective_scan(dev["x"], dev["dt"], dev["A"], dev["B"], dev["C"], D=dev["D"], z=dev["z"], conv_w=dev["conv_w"],
+                           a_geometric=True, seq_splits=16, workspace=ws)
+    check_blocks(to_np(y), run_ref(inp), "bf16", 16)
+
+
 @pytest.mark.parametrize("L", [63, 64, 191, 192, 400])
 def test_auto_plans_segments_of_default_calls(L):
     """Every choice left to the library, on both sides of the lengths where its plan changes."""

@@ -66,6 +66,22 @@ def test_noalloc_matches_workspace_variant_twice(dtype):
         assert torch.equal(got, want), f"call {call}: max diff {(got.float() - want.float()).abs().max().item()}"
 
 
+def test_noalloc_takes_what_its_own_plan_fits():
+    """700 steps in 16 segments are 11 segments of 64 steps here (6.9 MB of carries) and would be 15 in the look-back form's
+    plan (9.7 MB): the built-in array serves the first."""
+    import torch
+    from helixml_b200 import _lib as L, ops
+    inp = synth.scan_inputs(93, 10, 700, 1024, 16, 4, bf16=True)
+    dev = {k: to_dev(v, "bf16" if k in ("x", "dt", "z", "B", "C") else None) for k, v in inp.items()}
+    assert ops.scan_workspace_bytes(10, 700, 1024, torch.bfloat16, 16) > 8 << 20
+    want = ops.selective_scan(dev["x"], dev["dt"], dev["A"], dev["B"], dev["C"], D=dev["D"], z=dev["z"], conv_w=dev["conv_w"],
+                              variant=L.SCAN_SEQSPLIT, seq_splits=16, a_geometric=True)
+    got = torch.full_like(want, float("nan"))
+    a = _args(L, dev, got, L.HX_BF16, 16)
+    L.check(L.lib().hx_selective_scan_fwd_noalloc(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert torch.equal(got, want) and L.device_status() == 0
+
+
 def test_noalloc_rejects_oversized_problem():
     from helixml_b200 import _lib as L
     lib = L.lib()
