@@ -576,6 +576,30 @@ def test_workspace_sized_for_chained_segments_serves_auto():
     check_blocks(to_np(y), run_ref(inp), "bf16", 16)
 
 
+@pytest.mark.parametrize("geom", [True, False])
+@pytest.mark.parametrize("variant,splits,step", [(DIRECT, 0, 1.0), (TILED, 0, 1.0), (0, 3, 1.0 / 16)])
+def test_fp32_decays_keep_subnormal_results(geom, variant, splits, step):
+    """Decays of 1e-41 to 6e-39 (subnormal) times a state of 1e37: per step (one pass) and over a 16-step segment (the
+    aggregates and the fold of the look-back form).  exp(A dt) is good to |A dt| 2^-23 or the subnormal spacing."""
+    D, L = 32, 48
+    inp = synth.scan_inputs(67, 1, L, D, 16, 4, bf16=False)
+    inp["dt"][:] = np.log(np.expm1(step))
+    inp["B"][:] = inp["C"][:] = 1.0
+    inp["x"][:] = 0.0
+    inp["x"][:, [15, 16] if splits else [15]] = 1e37
+    a0 = -np.linspace(88.5, 94.0, D)
+    inp["A"] = (a0[:, None] * (np.arange(1, 17) if geom else np.linspace(1.0, 0.97, 16))).astype(np.float32)
+    got = run_gpu(inp, "f32", variant=variant, geom=geom, gate=False, skip=False, conv=False, seq_splits=splits)
+    h, want = np.zeros((D, 16)), np.zeros((L, D))
+    for t in range(L):
+        h = np.exp(inp["A"].astype(np.float64) * step) * h + step * inp["x"][0, t].astype(np.float64)[:, None]
+        want[t] = h.sum(1)
+    rows = slice(32, 36) if splits else slice(16, 17)
+    err = np.max(np.abs(got[0, rows] - want[rows]) / (np.abs(want[rows]) + 1e-30))
+    # per step of the look-back form: 100 * 2^-23 of the exponent and 1.4e-45 / 1e-41 of the subnormal spacing
+    assert np.all(want[32 if splits else 16] > 1e-6) and err <= 1e-3, err
+
+
 @pytest.mark.parametrize("L", [63, 64, 191, 192, 400])
 def test_auto_plans_segments_of_default_calls(L):
     """Every choice left to the library, on both sides of the lengths where its plan changes."""
