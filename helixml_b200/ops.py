@@ -133,7 +133,8 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, d
     a.reserved = tune
     auto = variant == L.SCAN_AUTO
     if a_geometric is None:
-        a.a_geometric = 2 if auto and N == 16 else (1 if check_geometric(A) else 0)
+        # 2 hands A to the kernel unseen, so it has to be device memory; the check on the host refuses anything else
+        a.a_geometric = 2 if auto and N == 16 and A.is_cuda else (1 if check_geometric(A) else 0)
     else:
         a.a_geometric = 1 if a_geometric else 0
     planned = auto and seq_splits == 0 and N == 16 and Bsz > 0 and Lq > 0 and Dm > 0
@@ -312,7 +313,7 @@ def mamba_block(x, w: dict, d_state: int, d_conv: int, workspace=None, scan_vari
     a.Dskip = _f32(w["D"]).data_ptr()
     # the scan's plan (and with it the workspace size) depends on the variant and on whether A is geometric
     a.scan_variant = scan_variant
-    if a_geometric is None and scan_variant == L.SCAN_AUTO and d_state == 16:
+    if a_geometric is None and scan_variant == L.SCAN_AUTO and d_state == 16 and w["A"].is_cuda:
         a.a_geometric = 2  # the kernel looks at A itself: no copy back, no synchronisation
     else:
         a.a_geometric = 1 if (check_geometric(w["A"]) if a_geometric is None else a_geometric) else 0

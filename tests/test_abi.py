@@ -137,3 +137,33 @@ def test_errors_are_thread_local():
     t.start()
     t.join()
     assert seen["msg"] == b"" and b"NULL" in lib.hx_last_error()
+
+
+def test_decays_in_host_memory_are_refused_before_the_launch(monkeypatch):
+    """A kernel that looks at A itself must not be given a host address: the check on the host, whose copy refuses it, runs
+    for an A that is not on the device."""
+    import torch
+    from helixml_b200 import ops
+
+    class Refused(Exception):
+        pass
+
+    def refuse(A):
+        raise Refused
+
+    monkeypatch.setattr(ops, "check_geometric", refuse)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops.L, "check", lambda status: None)
+
+    class NoLaunch:
+        def __getattr__(self, name):
+            return lambda *a: 0
+
+    monkeypatch.setattr(ops.L, "lib", NoLaunch)
+    x, bc, A = torch.zeros(1, 20, 32), torch.zeros(1, 20, 16), -torch.ones(32, 16)
+    with pytest.raises(Refused):
+        ops.selective_scan(x, x, A, bc, bc)
+    w = {"W_in": torch.zeros(64, 16), "W_x": torch.zeros(33, 32), "W_dt": torch.zeros(32, 1), "W_out": torch.zeros(16, 32),
+         "conv_w": torch.zeros(32, 4), "b_dt": torch.zeros(32), "A": A, "D": torch.zeros(32)}
+    with pytest.raises(Refused):
+        ops.mamba_block(torch.zeros(1, 20, 16), w, 16, 4)
