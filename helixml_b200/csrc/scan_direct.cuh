@@ -131,6 +131,13 @@ struct DirectCfg {
 // against 2.011e-7).
 template <bool FAST> __device__ __forceinline__ float decay_exp2(float x) { return FAST ? ex2_approx(x) : exp2f(x); }
 
+// The decay of a whole segment as the fold applies it to the state h.  Step by step, a zero state stays zero and an infinite
+// one infinite; the product of the steps' decays may have overflowed (A > 0) or underflowed, and 0 * inf would be a NaN.
+__device__ __forceinline__ float fold_decay(float a, float h) {
+    const float m = fabsf(h);
+    return m > 0.f && m < INFINITY ? a : 1.f;
+}
+
 template <typename T> __device__ __forceinline__ float2 ld_chan2(const char *p);  // two adjacent channels
 template <> __device__ __forceinline__ float2 ld_chan2<float>(const char *p) { return *reinterpret_cast<const float2 *>(p); }
 template <> __device__ __forceinline__ float2 ld_chan2<__nv_bfloat16>(const char *p) {
@@ -604,7 +611,8 @@ scan_direct_body(const CUtensorMap &tm_x, const CUtensorMap &tm_dt, const CUtens
                                 a[j] = make_float2(decay_exp2<FAST>(sd[f] * a2l[GEOM ? 0 : e][2 * j]), decay_exp2<FAST>(sd[f] * a2l[GEOM ? 0 : e][2 * j + 1]));
                         }
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) h[e][j] = fma2(a[j], h[e][j], qv[f][j]);
+                        for (int j = 0; j < 8; ++j)
+                            h[e][j] = fma2(make_float2(fold_decay(a[j].x, h[e][j].x), fold_decay(a[j].y, h[e][j].y)), h[e][j], qv[f][j]);
                     }
                 }
             }

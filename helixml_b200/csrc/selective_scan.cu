@@ -805,6 +805,9 @@ static hx_status launch_tiled_inst(const hx_scan_args *a, const TiledParams &p, 
     return check_launch("scan_tiled_kernel");
 }
 
+// 2 means that nobody has looked at A yet
+static bool asserted_geometric(const hx_scan_args *a) { return a->a_geometric != 0 && a->a_geometric != 2; }
+
 static int choose_lpc(const hx_scan_args *a) {
     if (a->lanes_per_channel == 1 || a->lanes_per_channel == 2 || a->lanes_per_channel == 4)
         return a->lanes_per_channel;
@@ -825,7 +828,7 @@ static hx_status launch_tiled(const hx_scan_args *a, bool split, cudaStream_t st
     // `reserved` picks another (chunk, stages) pair for the bf16 / geometric / standard path (tuning knob)
     const bool stdp0 = a->conv_w != nullptr && a->z != nullptr && a->dt_softplus != 0;
     // only 1 and 2 name a tuning variant; anything else (the direct kernel's selector among them) is the default
-    const int tune = (bf && a->a_geometric == 1 && stdp0 && (a->reserved == 1 || a->reserved == 2)) ? a->reserved : 0;
+    const int tune = (bf && asserted_geometric(a) && stdp0 && (a->reserved == 1 || a->reserved == 2)) ? a->reserved : 0;
     const int ES = bf ? 2 : 4, DT = 128 / ES, TC = tune >= 1 ? 16 : (bf ? kChunkBf16 : kChunkF32);
     const int tiles = (a->d_inner + DT - 1) / DT;
     int n_seg = 1, seg_len = (a->seq_len + TC - 1) / TC * TC;
@@ -887,7 +890,7 @@ static hx_status launch_tiled(const hx_scan_args *a, bool split, cudaStream_t st
                a->batch, n_seg);
     dim3 grid(tiles, a->batch, n_seg);
     const int lpc = choose_lpc(a);
-    const bool geom = a->a_geometric == 1;  // (2, decided on the device, is the one-lane-per-channel kernel's)
+    const bool geom = asserted_geometric(a);  // (2, decided on the device, is the one-lane-per-channel kernel's)
     // the standard path (4-tap conv, softplus, gate) has its flags fixed at compile time
     const bool stdp = a->conv_w != nullptr && a->z != nullptr && a->dt_softplus != 0;
 #define HX_TILED_CASE(T, LPC, GEOM, TCv, ST)                                                    \
@@ -994,6 +997,11 @@ static bool lookback_ok(const hx_scan_args *a) {
     if (a->W_dt) return a->conv_w == nullptr && a->z != nullptr && a->dt_softplus != 0;
     return true;
 }
+
+// Whether AUTO may look back.  The form multiplies a state by exp(A * sum of dt), which stands for the product of the
+// steps' decays as long as they do not grow: softplus makes dt >= 0.  Without it dt may be negative, the product of a
+// segment overflows where the steps' own do not, and only a caller who asserts A and asks for segments gets the form.
+static bool auto_lookback_ok(const hx_scan_args *a) { return lookback_ok(a) && (a->dt_softplus != 0 || asserted_geometric(a)); }
 
 // hx_debug_scan_orphan_segment: first segment the calling thread's next chained launch starts (0 = all of them)
 static thread_local int t_orphan_from = 0;
@@ -1159,7 +1167,7 @@ static hx_status launch_direct(const hx_scan_args *a, bool split, cudaStream_t s
 // a second warp: [12, 1024, 2048] 348 / 365, [6, 1500, 2048] 447 / 277.
 static double warps_per_sm(const hx_scan_args *a) { return (double)a->batch * a->d_inner / 32.0 / sm_count(); }
 static bool one_pass_pays(const hx_scan_args *a) {
-    const double limit = a->io_dtype != HX_BF16 ? 4.0 : a->a_geometric == 1 ? 2.5 : 3.0;
+    const double limit = a->io_dtype != HX_BF16 ? 4.0 : asserted_geometric(a) ? 2.5 : 3.0;
     return warps_per_sm(a) >= limit;
 }
 // Sequences this short are over before a second launch starts: one pass (bf16) or the lane-split kernel (fp32, general A).
@@ -1170,7 +1178,7 @@ int auto_channels_per_lane(const hx_scan_args *a) { return choose_cpl(a); }
 
 ScanKind auto_kind(const hx_scan_args *a) {
     if (one_pass_pays(a)) return ScanKind::Direct;
-    if (a->seq_splits > 1 && lookback_ok(a)) return ScanKind::LookBack;
+    if (a->seq_splits > 1 && auto_lookback_ok(a)) return ScanKind::LookBack;
     if (a->W_dt != nullptr) return ScanKind::Direct;  // the fused dt projection exists only there
     if (a->io_dtype == HX_BF16 && a->a_geometric != 0) return ScanKind::Direct;
     return ScanKind::Tiled;
@@ -1178,7 +1186,7 @@ ScanKind auto_kind(const hx_scan_args *a) {
 
 // Sequence segments for AUTO.
 int auto_splits(const hx_scan_args *a) {
-    if (!one_pass_pays(a) && !a->z_is_gate) {
+    if (!one_pass_pays(a) && auto_lookback_ok(a)) {
         // look-back form: as many segments as fill the three CTAs an SM holds once (one more and some SMs run a fourth
         // after the others: [3, 1631, 1536] with 10 / 16 segments 3.39 / 3.28 ms a model pass, 12 fill 432 of 444 slots), of
         // at least 32 steps (16 where the sequence has few)

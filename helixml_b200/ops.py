@@ -76,7 +76,7 @@ def suggest_splits(batch, seq_len, d_inner, dtype, a_geometric=True) -> int:
     a = L.ScanArgs()
     a.batch, a.seq_len, a.d_inner, a.d_state = batch, seq_len, d_inner, 16
     a.io_dtype = L.HX_BF16 if dtype == torch.bfloat16 else L.HX_F32
-    a.a_geometric = 1 if a_geometric else 0
+    a.a_geometric, a.dt_softplus = (1 if a_geometric else 0), 1
     return int(L.lib().hx_selective_scan_suggest_splits(C.byref(a)))
 
 
@@ -86,7 +86,8 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, d
     """Fused selective scan (hx_selective_scan_fwd).  x, dt, z, y: [B, L, D]; Bm, Cm: [B, L, N].
     z_is_gate: z already holds silu(z).
     With every choice left open (SCAN_AUTO, seq_splits 0) the library plans the sequence segments, and a_geometric=None
-    leaves it to the kernel to look at A: no device-to-host copy, no synchronisation."""
+    leaves it to the kernel to look at A: no device-to-host copy, no synchronisation.  A ready-made gate, or a dt that is
+    used as it is (and may be negative), takes one pass, whose kernel wants to know A beforehand."""
     Bsz, Lq, Dm = x.shape
     N = A.shape[1]
     y = out if out is not None else torch.empty((Bsz, Lq, Dm), dtype=x.dtype, device=x.device)
@@ -131,7 +132,7 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, d
     a.z_is_gate = 1 if z_is_gate else 0
     a.lanes_per_channel = lanes_per_channel
     a.reserved = tune
-    auto = variant == L.SCAN_AUTO
+    auto = variant == L.SCAN_AUTO and dt_softplus and not z_is_gate
     if a_geometric is None:
         # 2 hands A to the kernel unseen, so it has to be device memory; the check on the host refuses anything else
         a.a_geometric = 2 if auto and N == 16 and A.is_cuda else (1 if check_geometric(A) else 0)

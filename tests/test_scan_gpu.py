@@ -600,6 +600,45 @@ def test_fp32_decays_keep_subnormal_results(geom, variant, splits, step):
     assert np.all(want[32 if splits else 16] > 1e-6) and err <= 1e-3, err
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("geom", [None, True, False])
+@pytest.mark.parametrize("decay", [-1.0, 2.0])
+def test_growing_states_that_are_still_zero(dtype, geom, decay):
+    """A product of decays that overflows over a segment, on states that are zero until the last steps: a negative dt used
+    as it is, and a positive A.  The result is what the recurrence gives step by step, not 0 * inf."""
+    D, L = 96, 300
+    inp = synth.scan_inputs(68, 1, L, D, 16, 4, bf16=dtype == "bf16")
+    inp["A"] = np.ascontiguousarray(np.broadcast_to(decay * np.arange(1, 17, dtype=np.float32), (D, 16)))
+    if decay > 0 and geom:
+        geom = False  # positive decays are not what a caller may assert
+    inp["x"][:, :297] = 0.0
+    softplus = decay > 0
+    inp["dt"][:] = 1.0 if softplus else -1.0
+    kw = dict(gate=False, skip=False, conv=False, softplus=softplus)
+    got, hg = run_gpu(inp, dtype, variant=0, geom=geom, state=True, **kw)
+    ref, hr = run_ref(inp, state=True, **kw)
+    assert np.all(np.isfinite(ref)) and np.all(got[:, :297] == 0)
+    check(got / 1e3, ref / 1e3, dtype)  # states of up to e^(2 * 16 * 2.6)
+    assert np.all(np.isfinite(hg))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_infinite_state_stays_infinite_in_the_lookback_form(dtype):
+    """An infinite input early on, general A: the states it reaches stay infinite over the segments that follow, whose decays
+    underflow to zero, as they do step by step."""
+    D, L = 96, 300
+    inp = synth.scan_inputs(69, 1, L, D, 16, 4, bf16=dtype == "bf16")
+    inp["A"] = -np.exp(synth.uniform(69, "Alog", (D, 16), 0.0, 2.0)).astype(np.float32)
+    inp["dt"][:] = 1.0
+    inp["B"][:] = inp["C"][:] = 1.0
+    inp["x"][:, 5, ::2] = np.inf
+    kw = dict(gate=False, skip=False, conv=False)
+    for geom in (None, False):
+        got, hg = run_gpu(inp, dtype, variant=0, geom=geom, state=True, **kw)
+        assert np.all(np.isposinf(got[:, 6:, ::2])) and np.all(np.isposinf(hg[:, ::2]))
+        assert np.all(np.isfinite(got[:, :, 1::2]))
+
+
 @pytest.mark.parametrize("L", [63, 64, 191, 192, 400])
 def test_auto_plans_segments_of_default_calls(L):
     """Every choice left to the library, on both sides of the lengths where its plan changes."""
