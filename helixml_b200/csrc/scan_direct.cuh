@@ -573,6 +573,21 @@ scan_direct_body(const CUtensorMap &tm_x, const CUtensorMap &tm_dt, const CUtens
                 if (dch + e >= p.D) continue;
                 const int64_t c0 = (int64_t)b * p.D + dch + e, cs = (int64_t)p.B * p.D;
                 const float2 *q0 = reinterpret_cast<const float2 *>(p.carry + c0 * 16);
+                auto segment_decays = [&](float sdt, float2 (&a)[8]) {
+                    if constexpr (GEOM) {
+                        const float r = decay_exp2<FAST>(sdt * a0_[e]);
+                        a[0] = make_float2(r, r * r);
+                        a[1] = mul2(a[0], splat2(a[0].y));
+                        a[2] = mul2(a[0], splat2(a[1].y));
+                        a[3] = mul2(a[1], splat2(a[1].y));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) a[4 + j] = mul2(a[j], splat2(a[3].y));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            a[j] = make_float2(decay_exp2<FAST>(sdt * a2l[GEOM ? 0 : e][2 * j]), decay_exp2<FAST>(sdt * a2l[GEOM ? 0 : e][2 * j + 1]));
+                    }
+                };
 #pragma unroll
                 for (int j = 0; j < 8; ++j) h[e][j] = q0[j];  // segment 0 starts from zero: its aggregate is its end state
                 // Four aggregates are fetched before the first is used: one at a time a segment with many predecessors
@@ -597,22 +612,27 @@ scan_direct_body(const CUtensorMap &tm_x, const CUtensorMap &tm_dt, const CUtens
                     for (int f = 0; f < FB; ++f) {
                         if (js + f >= seg) break;
                         float2 a[8];
-                        if constexpr (GEOM) {
-                            const float r = decay_exp2<FAST>(sd[f] * a0_[e]);
-                            a[0] = make_float2(r, r * r);
-                            a[1] = mul2(a[0], splat2(a[0].y));
-                            a[2] = mul2(a[0], splat2(a[1].y));
-                            a[3] = mul2(a[1], splat2(a[1].y));
+                        segment_decays(sd[f], a);
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) a[4 + j] = mul2(a[j], splat2(a[3].y));
-                        } else {
+                        for (int j = 0; j < 8; ++j) h[e][j] = fma2(a[j], h[e][j], qv[f][j]);
+                    }
+                }
+                // A state that comes out infinite or NaN is folded again with fold_decay, which on every fold would cost the
+                // short look-backs 3 to 17 % (bf16 [3, 1111, 640]: 27.3 -> 31.4 us).
+                float2 fin = make_float2(0.f, 0.f);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                a[j] = make_float2(decay_exp2<FAST>(sd[f] * a2l[GEOM ? 0 : e][2 * j]), decay_exp2<FAST>(sd[f] * a2l[GEOM ? 0 : e][2 * j + 1]));
-                        }
+                for (int j = 0; j < 8; ++j) fin = fma2(h[e][j], make_float2(0.f, 0.f), fin);
+                if (!(fin.x + fin.y == 0.f)) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) h[e][j] = q0[j];
+#pragma unroll 1
+                    for (int js = 1; js < seg; ++js) {
+                        float2 a[8];
+                        segment_decays(p.sdt[c0 + js * cs], a);
+                        const float2 *qj = reinterpret_cast<const float2 *>(p.carry + (c0 + js * cs) * 16);
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
-                            h[e][j] = fma2(make_float2(fold_decay(a[j].x, h[e][j].x), fold_decay(a[j].y, h[e][j].y)), h[e][j], qv[f][j]);
+                            h[e][j] = fma2(make_float2(fold_decay(a[j].x, h[e][j].x), fold_decay(a[j].y, h[e][j].y)), h[e][j], qj[j]);
                     }
                 }
             }
