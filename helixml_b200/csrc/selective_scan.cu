@@ -1171,22 +1171,47 @@ static bool one_pass_pays(const hx_scan_args *a) {
     return warps_per_sm(a) >= limit;
 }
 // Sequences this short are over before a second launch starts: one pass (bf16) or the lane-split kernel (fp32, general A).
-// Measured at 1 x 100 x 1536: bf16 12.5 us in one pass; fp32 18.7 us lane-split against 25 us in the look-back form.
-static bool short_sequence(const hx_scan_args *a) { return a->seq_len < (a->io_dtype == HX_BF16 ? 64 : 192); }
+// Measured, us, short form / look-back: bf16 [1, 64, 1536] general A 9.7 / 10.5, [1, 100, 1536] 14.6 / 14.4; fp32 [1, 192, 256]
+// geometric 24.4 / 22.4, general 27.2 / 33, [1, 256, 1536] general 35.7 / 34.5.
+static bool short_sequence(const hx_scan_args *a) {
+    if (a->io_dtype == HX_BF16) return a->seq_len < (a->a_geometric == 0 ? 80 : 64);
+    return a->seq_len < (a->a_geometric == 0 ? 256 : 192);
+}
+// fp32: whether the look-back form beats the lane-split kernel in one pass.  The look-back form's time a step goes with the
+// warps there are (0.08 us a step for each warp per SM with a geometric A, 0.12 to 0.14 with 16 exp2f a point); the lane-split
+// kernel takes 0.14 us a step with four lanes a channel and about 0.25 with two (choose_lpc) whatever there is of them.
+// Measured, us, look-back / lane-split: geometric [4, 2048, 1536] 192 / 287, [8, 512, 1024] 76.5 / 71.8, [6, 1500, 2048] 277 / 332;
+// general [8, 512, 512] 64 / 69, [4, 300, 1536] 57 / 49, [4, 2048, 1536] 322 / 309, [8, 512, 1024] 119 / 79, [10, 2000, 1024] 510 / 539,
+// [6, 1500, 2048] 444 / 410, [8, 512, 2048] 201 / 273 (there the lane-split kernel needs a second wave of its 32-channel CTAs).
+// An A that nobody has looked at (2) the lane-split kernel takes as general, so the line lies higher for it.
+static bool lookback_beats_lanes(const hx_scan_args *a) {
+    const double w = warps_per_sm(a);
+    const bool one_wave = (double)a->batch * ((a->d_inner + 31) / 32) <= 3.0 * sm_count();
+    const double lanes = (w < 2.0 ? 1.0 : 1.8) * (one_wave ? 1.0 : 2.0);
+    const double look = (asserted_geometric(a) ? 0.58 : a->a_geometric == 2 ? 0.65 : 0.82) * w;
+    return look < lanes;
+}
 
 int auto_channels_per_lane(const hx_scan_args *a) { return choose_cpl(a); }
 
+static bool auto_looks_back(const hx_scan_args *a) {
+    if (one_pass_pays(a) || !auto_lookback_ok(a)) return false;
+    // (with segments asked for, the lane-split kernel would chain them, which only costs it)
+    return a->io_dtype == HX_BF16 || (a->seq_splits > 1 && asserted_geometric(a)) || lookback_beats_lanes(a);
+}
+
 ScanKind auto_kind(const hx_scan_args *a) {
     if (one_pass_pays(a)) return ScanKind::Direct;
-    if (a->seq_splits > 1 && auto_lookback_ok(a)) return ScanKind::LookBack;
+    if (a->seq_splits > 1 && auto_looks_back(a)) return ScanKind::LookBack;
     if (a->W_dt != nullptr) return ScanKind::Direct;  // the fused dt projection exists only there
-    if (a->io_dtype == HX_BF16 && a->a_geometric != 0) return ScanKind::Direct;
+    // (without softplus the one-lane-per-channel kernel tests its flags at run time: 5 to 9 % behind the lane-split kernel)
+    if (a->io_dtype == HX_BF16 && a->a_geometric != 0 && a->dt_softplus) return ScanKind::Direct;
     return ScanKind::Tiled;
 }
 
 // Sequence segments for AUTO.
 int auto_splits(const hx_scan_args *a) {
-    if (!one_pass_pays(a) && auto_lookback_ok(a)) {
+    if (auto_looks_back(a)) {
         // look-back form: as many segments as fill the three CTAs an SM holds once (one more and some SMs run a fourth
         // after the others: [3, 1631, 1536] with 10 / 16 segments 3.39 / 3.28 ms a model pass, 12 fill 432 of 444 slots), of
         // at least 32 steps (16 where the sequence has few)
@@ -1200,6 +1225,7 @@ int auto_splits(const hx_scan_args *a) {
     // or far above the slots of the device (about 3 CTAs per SM), and the fp32 form only loses by the hand-overs.
     const int tile = one_pass_pays(a) ? 128 : (a->io_dtype == HX_BF16 ? 64 : 32);
     const double ctas = (double)a->batch * ((a->d_inner + tile - 1) / tile), slots = 3.0 * sm_count();
+    if (a->io_dtype != HX_BF16 && !one_pass_pays(a) && auto_lookback_ok(a)) return 1;  // the lane-split kernel, in one pass
     if (ctas >= 8.0 * slots || ctas <= sm_count() || (a->io_dtype != HX_BF16 && one_pass_pays(a))) return 1;
     int s = (int)(HX_SCAN_CHAIN_WAVES * slots / ctas + 0.999);
     if (s > 8) s = 8;                                      // 8 segments: within 2 % of the best at every shape measured

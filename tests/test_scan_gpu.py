@@ -600,6 +600,18 @@ def test_fp32_decays_keep_subnormal_results(geom, variant, splits, step):
     assert np.all(want[32 if splits else 16] > 1e-6) and err <= 1e-3, err
 
 
+@pytest.mark.parametrize("geom", [None, True, False])
+@pytest.mark.parametrize("B,L,D", [(4, 100, 1536), (8, 280, 1024), (6, 300, 2048), (8, 257, 2048), (1, 255, 64), (1, 256, 64)])
+def test_fp32_default_calls_on_both_sides_of_the_lookback_rule(geom, B, L, D):
+    inp = synth.scan_inputs(70, B, L, D, 16, 4, bf16=False)
+    if geom is not True:
+        inp["A"] = (inp["A"] * np.exp(synth.uniform(70, "f", (D, 16), -0.3, 0.3))).astype(np.float32)
+    got, hg = run_gpu(inp, "f32", variant=0, geom=geom, state=True)
+    ref, hr = run_ref(inp, state=True)
+    check_blocks(got, ref, "f32", 64, 128)
+    check(hg, hr, "f32")
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("geom", [None, True, False])
 @pytest.mark.parametrize("decay", [-1.0, 2.0])
