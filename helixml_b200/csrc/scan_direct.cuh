@@ -103,8 +103,12 @@ struct DirectCfg {
     static constexpr int UNROLL = HX_SCAN_UNROLL;
     static constexpr bool FULL = FUSEDT_ == 2 || (HX_SCAN_FULL_UNROLL && CPL_ == 1);   // whole chunks fully unrolled
     static constexpr int REM_UNROLL = FULL ? 1 : HX_SCAN_UNROLL;                       // the loop they do not take
-    // with a general A the unrolled chunk would take 250 registers (the exponentials of many steps in flight), one CTA per SM
-    static constexpr int MIN_CTAS = GEOM_ != 1 ? (CPL_ == 2 ? 2 : MODE_ != 0 ? HX_SCAN_MINB_GENERAL : 3)
+    // With a general A the unrolled chunk takes 250 registers (the exponentials of many steps in flight), one CTA per SM, if
+    // nothing holds it back.  bf16 in one pass: held to two CTAs ([8, 512, 2048] 63 us against 66 unheld and 74 held to three,
+    // [16, 2048, 1536] 361 against 436 held to three); fp32 in one pass to three ([3, 1111, 640] 404 against 440 held to two or
+    // unheld).
+    static constexpr int MIN_CTAS_GENERAL = CPL_ == 2 ? 2 : MODE_ != 0 ? HX_SCAN_MINB_GENERAL : sizeof(T) == 2 ? 2 : 3;
+    static constexpr int MIN_CTAS = GEOM_ != 1 ? MIN_CTAS_GENERAL
                                     : (MODE_ != 0 && !FUSEDT_) ? HX_SCAN_MINB_LOOKBACK : HX_SCAN_MINB_CHAINED;
     static constexpr int X_BYTES = (TC + 3) * 128;
     static constexpr int ROW_BYTES = TC * 128;
