@@ -16,7 +16,7 @@ template <int EPI> __device__ __forceinline__ float apply_epilogue(float v) {
 }
 
 // The few-rows kernel (gemm_skinny.cu): M <= 64, K a multiple of 32, operands 16-byte aligned with row strides
-// that are multiples of 8 elements.  `chain`: see launch_chained.
+// that are multiples of 8 elements.  `chain` (no activation): see launch_chained.
 hx_status launch_skinny(const void *A, int64_t lda, const void *W, int64_t ldw, const float *bias, void *C, int64_t ldc,
                         int c_dtype, int M, int N, int K, int epi, int epi_col0, cudaStream_t st, bool chain = false);
 

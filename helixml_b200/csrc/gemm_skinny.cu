@@ -10,8 +10,13 @@
 // long as A and B agree, so inside a block of 32 k values lane (g, tid) loads the 8 consecutive elements
 // k = 8 tid .. 8 tid + 7 of its row and uses them as the two k-halves of two MMAs:
 //   MMA j (j = 0, 1): "k pair 2 tid" = elements 4 j + {0, 1}, "k pair 2 tid + 8" = elements 4 j + {2, 3}.
-// A comes straight from global memory (it is M x K, a few tens of KB, shared by every CTA through L2/L1).  A, C and the bias
-// carry no __restrict__: their loads must stay behind chain_wait().
+// A comes straight from global memory (it is M x K, a few tens of KB, shared by every CTA through L2/L1).
+//
+// CHAIN: launched by launch_chained under the kernel before it.  A, C and the bias then carry no __restrict__ (their loads must
+// stay behind chain_wait()) and the weights of four k-blocks, inner dimensions up to 2048, are requested before waiting.  By
+// itself the kernel has nothing to fetch them under and takes two blocks a trip, W and A of one before the other's: four of W
+// first cost registers that more rows need and put the rows behind them (17 x 4096 x 4096 16.9 us against 10.9, 24 x 4096 x 1024
+// 7.2 against 5.4, 32 x 3072 x 768 6.0 against 5.2, 1 x 4096 x 4096 7.5 against 6.6).
 #include "gemm.cuh"
 
 namespace hx {
@@ -19,11 +24,11 @@ namespace gemm {
 
 constexpr int kSkinnyWarps = 16;
 
-template <int MT, typename TC, int EPI>
-__global__ void __launch_bounds__(kSkinnyWarps * 32)
-gemm_skinny_kernel(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *__restrict__ W, int64_t ldw,
-                   const float *bias, TC *C, int64_t ldc, int M, int N, int K, int epi_col0) {
-    chain_trigger();
+template <int MT, typename TC, int EPI, bool CHAIN>
+__device__ __forceinline__ void
+gemm_skinny_body(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *W, int64_t ldw, const float *bias, TC *C, int64_t ldc,
+                 int M, int N, int K, int epi_col0) {
+    if constexpr (CHAIN) chain_trigger();
     __shared__ float partial[kSkinnyWarps * MT * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tid = lane & 3;
@@ -48,48 +53,58 @@ gemm_skinny_kernel(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *__r
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[mt][i] = 0.f;
 
-    // this warp's k-blocks: warp, warp + 16, ...  Four blocks of W per trip (inner dimensions up to 2048 in one), A two
-    // blocks at a time.  W does not depend on the kernel before this one, so the first trip's are requested before waiting.
-    uint4 b[4];
-    auto fetch_w = [&](int k0) {
+    auto mma = [&](const uint4 (&a)[MT][2], const uint4 &b) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u * kSkinnyWarps * 32;
-            b[u] = (n_ok && k < K) ? *reinterpret_cast<const uint4 *>(wrow + k) : zero4;
+        for (int mt = 0; mt < MT; ++mt) {
+            // fragment registers: a0 = (row g, k pair), a1 = (row g+8, k pair), a2 = (row g, k pair + 8), a3 = (row g+8, ...)
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                         "{%0, %1, %2, %3};"
+                         : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                         : "r"(a[mt][0].x), "r"(a[mt][1].x), "r"(a[mt][0].y), "r"(a[mt][1].y), "r"(b.x), "r"(b.y));
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                         "{%0, %1, %2, %3};"
+                         : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                         : "r"(a[mt][0].z), "r"(a[mt][1].z), "r"(a[mt][0].w), "r"(a[mt][1].w), "r"(b.z), "r"(b.w));
         }
     };
-    fetch_w(warp * 32);
-    chain_wait();
-    for (int k0 = warp * 32; k0 < K; k0 += kSkinnyWarps * 128) {
-        if (k0 != warp * 32) fetch_w(k0);
+    // this warp's k-blocks: warp, warp + 16, ...
+    constexpr int STEP = kSkinnyWarps * 32;
+    auto ld_w = [&](int k) { return (n_ok && k < K) ? *reinterpret_cast<const uint4 *>(wrow + k) : zero4; };
+    auto ld_a = [&](uint4 (&a)[MT][2], int k) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            if (k0 + half * kSkinnyWarps * 64 >= K) break;   // warp-uniform
-            uint4 a[2][MT][2];
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) a[mt][h] = (a_ok[mt][h] && k < K) ? *reinterpret_cast<const uint4 *>(arow[mt][h] + k) : zero4;
+    };
+    uint4 a[2][MT][2];
+    if constexpr (!CHAIN) {  // two blocks per trip so that their loads overlap
+        for (int k0 = warp * 32; k0 < K; k0 += 2 * STEP) {
+            uint4 b[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const int k = k0 + (half * 2 + u) * kSkinnyWarps * 32;
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        a[u][mt][h] = (a_ok[mt][h] && k < K) ? *reinterpret_cast<const uint4 *>(arow[mt][h] + k) : zero4;
+                b[u] = ld_w(k0 + u * STEP);
+                ld_a(a[u], k0 + u * STEP);
             }
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const uint4 bu = b[half * 2 + u];
+            for (int u = 0; u < 2; ++u) mma(a[u], b[u]);
+        }
+    } else {                 // four of W, the first trip's before the wait, and twice two of A
+        uint4 b[4];
+        auto fetch_w = [&](int k0) {
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    // fragment registers: a0 = (row g, k pair), a1 = (row g+8, k pair), a2 = (row g, k pair + 8), a3 = (row g+8, ...)
-                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                                 "{%0, %1, %2, %3};"
-                                 : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
-                                 : "r"(a[u][mt][0].x), "r"(a[u][mt][1].x), "r"(a[u][mt][0].y), "r"(a[u][mt][1].y), "r"(bu.x), "r"(bu.y));
-                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                                 "{%0, %1, %2, %3};"
-                                 : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
-                                 : "r"(a[u][mt][0].z), "r"(a[u][mt][1].z), "r"(a[u][mt][0].w), "r"(a[u][mt][1].w), "r"(bu.z), "r"(bu.w));
-                }
+            for (int u = 0; u < 4; ++u) b[u] = ld_w(k0 + u * STEP);
+        };
+        fetch_w(warp * 32);
+        chain_wait();
+        for (int k0 = warp * 32; k0 < K; k0 += 4 * STEP) {
+            if (k0 != warp * 32) fetch_w(k0);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                if (k0 + half * 2 * STEP >= K) break;   // warp-uniform
+#pragma unroll
+                for (int u = 0; u < 2; ++u) ld_a(a[u], k0 + (half * 2 + u) * STEP);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) mma(a[u], b[half * 2 + u]);
             }
         }
     }
@@ -114,6 +129,19 @@ gemm_skinny_kernel(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *__r
     }
 }
 
+template <int MT, typename TC, int EPI>
+__global__ void __launch_bounds__(kSkinnyWarps * 32)
+gemm_skinny_kernel(const __nv_bfloat16 *__restrict__ A, int64_t lda, const __nv_bfloat16 *__restrict__ W, int64_t ldw,
+                   const float *__restrict__ bias, TC *__restrict__ C, int64_t ldc, int M, int N, int K, int epi_col0) {
+    gemm_skinny_body<MT, TC, EPI, false>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi_col0);
+}
+template <int MT, typename TC, int EPI>
+__global__ void __launch_bounds__(kSkinnyWarps * 32)
+gemm_skinny_chain_kernel(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *__restrict__ W, int64_t ldw, const float *bias,
+                         TC *C, int64_t ldc, int M, int N, int K, int epi_col0) {
+    gemm_skinny_body<MT, TC, EPI, true>(A, lda, W, ldw, bias, C, ldc, M, N, K, epi_col0);
+}
+
 template <int MT, typename TC>
 static hx_status launch_skinny_epi(const void *A, int64_t lda, const void *W, int64_t ldw, const float *bias, void *C, int64_t ldc,
                                    int M, int N, int K, int epi, int epi_col0, cudaStream_t st, bool chain) {
@@ -121,17 +149,27 @@ static hx_status launch_skinny_epi(const void *A, int64_t lda, const void *W, in
     auto a = static_cast<const __nv_bfloat16 *>(A), w = static_cast<const __nv_bfloat16 *>(W);
     auto c = static_cast<TC *>(C);
     cudaError_t e = cudaSuccess;
+#define HX_SKINNY_LAUNCH(KERNEL, EPI) e = launch_chained(chain, KERNEL<MT, TC, EPI>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0)
+    HX_REQUIRE(!chain || epi == kEpiNone || epi == kEpiAccumulate, HX_ERR_INVALID_INPUT, "a chained launch has no epilogue %d", epi);
     switch (epi) {
-        case kEpiNone: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiNone>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSilu: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSilu>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSoftplus: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSoftplus>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
-        case kEpiSiluFast: e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiSiluFast>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0); break;
+        case kEpiNone:
+            if (chain) HX_SKINNY_LAUNCH(gemm_skinny_chain_kernel, kEpiNone);
+            else HX_SKINNY_LAUNCH(gemm_skinny_kernel, kEpiNone);
+            break;
+        case kEpiSilu: HX_SKINNY_LAUNCH(gemm_skinny_kernel, kEpiSilu); break;
+        case kEpiSoftplus: HX_SKINNY_LAUNCH(gemm_skinny_kernel, kEpiSoftplus); break;
+        case kEpiSiluFast: HX_SKINNY_LAUNCH(gemm_skinny_kernel, kEpiSiluFast); break;
         case kEpiAccumulate:
-            if constexpr (sizeof(TC) == 4) e = launch_chained(chain, gemm_skinny_kernel<MT, TC, kEpiAccumulate>, grid, block, st, a, lda, w, ldw, bias, c, ldc, M, N, K, epi_col0);
-            else return fail(HX_ERR_DTYPE_MISMATCH, "accumulating GEMM needs an fp32 C");
+            if constexpr (sizeof(TC) == 4) {
+                if (chain) HX_SKINNY_LAUNCH(gemm_skinny_chain_kernel, kEpiAccumulate);
+                else HX_SKINNY_LAUNCH(gemm_skinny_kernel, kEpiAccumulate);
+            } else {
+                return fail(HX_ERR_DTYPE_MISMATCH, "accumulating GEMM needs an fp32 C");
+            }
             break;
         default: return fail(HX_ERR_INVALID_INPUT, "unknown epilogue %d", epi);
     }
+#undef HX_SKINNY_LAUNCH
     HX_CUDA(e);
     return check_launch("gemm_skinny_kernel");
 }
