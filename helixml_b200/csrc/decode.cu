@@ -147,25 +147,157 @@ conv_state_kernel(const T *__restrict__ x, int64_t xb, int64_t xr, T *__restrict
 //   A = rmsnorm(residual) * norm_w is formed on the fly from the fp32 residual stream (the row scale 1/rms is
 //   applied to the accumulators at the end, the sum of squares is gathered while the row is read);
 //   columns n < E get the conv step (window in, u out, window shifted), columns n >= E are z.
-// Work split as in gemm_skinny_kernel: 8 output columns per CTA, 8 warps share K in blocks of 32 (with 16 warps a CTA took
-// so many registers that the 384 CTAs of a 768-wide model did not fit the device at once), mma.sync with
+// Work split as in gemm_skinny_kernel: 8 output columns per CTA, 16 warps share K in blocks of 32, mma.sync with
 // the k-permuted 8-element operand loads, partial tiles summed through shared memory.
-constexpr int kStepWarps = 8;
+constexpr int kStepWarps = 16;
 
+template <int MT, bool CHAIN>
+__device__ __forceinline__ void
+inproj_step_body(const float *resid, const float *norm_w, float eps, const __nv_bfloat16 *W, __nv_bfloat16 *conv_state,
+                 const float *cw, const float *cb, __nv_bfloat16 *u, __nv_bfloat16 *z, int M, int K, int E, int Kc) {
+    if constexpr (CHAIN) {
+        chain_trigger();
+        chain_wait();
+    }
+    __shared__ float partial[kStepWarps * MT * 128];
+    __shared__ float ssq_part[kStepWarps][MT * 16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, tid = lane & 3;
+    const int n0 = blockIdx.x * 8;
+    const int n = n0 + g;  // the W row this lane loads (2E is a multiple of 8)
+    const __nv_bfloat16 *wrow = W + (int64_t)n * K + tid * 8;
+    float acc[MT][4], ssq[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        ssq[mt][0] = ssq[mt][1] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[mt][i] = 0.f;
+    }
+    for (int k0 = warp * 32; k0 < K; k0 += kStepWarps * 32) {
+        const uint4 b = *reinterpret_cast<const uint4 *>(wrow + k0);
+        const float4 w0 = *reinterpret_cast<const float4 *>(norm_w + k0 + tid * 8);
+        const float4 w1 = *reinterpret_cast<const float4 *>(norm_w + k0 + tid * 8 + 4);
+        uint4 a[MT][2];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = mt * 16 + h * 8 + g;
+                float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+                if (r < M) {
+                    const float *xr = resid + (int64_t)r * K + k0 + tid * 8;
+                    x0 = *reinterpret_cast<const float4 *>(xr);
+                    x1 = *reinterpret_cast<const float4 *>(xr + 4);
+                }
+                ssq[mt][h] += x0.x * x0.x + x0.y * x0.y + x0.z * x0.z + x0.w * x0.w + x1.x * x1.x + x1.y * x1.y +
+                              x1.z * x1.z + x1.w * x1.w;
+                const __nv_bfloat162 p0 = __floats2bfloat162_rn(x0.x * w0.x, x0.y * w0.y);
+                const __nv_bfloat162 p1 = __floats2bfloat162_rn(x0.z * w0.z, x0.w * w0.w);
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(x1.x * w1.x, x1.y * w1.y);
+                const __nv_bfloat162 p3 = __floats2bfloat162_rn(x1.z * w1.z, x1.w * w1.w);
+                a[mt][h] = make_uint4(*reinterpret_cast<const uint32_t *>(&p0), *reinterpret_cast<const uint32_t *>(&p1),
+                                      *reinterpret_cast<const uint32_t *>(&p2), *reinterpret_cast<const uint32_t *>(&p3));
+            }
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                         "{%0, %1, %2, %3};"
+                         : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                         : "r"(a[mt][0].x), "r"(a[mt][1].x), "r"(a[mt][0].y), "r"(a[mt][1].y), "r"(b.x), "r"(b.y));
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                         "{%0, %1, %2, %3};"
+                         : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                         : "r"(a[mt][0].z), "r"(a[mt][1].z), "r"(a[mt][0].w), "r"(a[mt][1].w), "r"(b.z), "r"(b.w));
+        }
+    }
+    // sums of squares: the four lanes of a row group hold different k, then the warps hold different k-blocks
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float v = ssq[mt][h];
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (tid == 0) ssq_part[warp][mt * 16 + h * 8 + g] = v;
+        }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+        *reinterpret_cast<float4 *>(&partial[((warp * MT + mt) * 32 + lane) * 4]) =
+            make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t >= MT * 128) return;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kStepWarps; ++w) v += partial[w * MT * 128 + t];
+    const int mt = t >> 7, ln = (t & 127) >> 2, i = t & 3;
+    const int r = mt * 16 + (i >> 1) * 8 + (ln >> 2);
+    const int c = n0 + 2 * (ln & 3) + (i & 1);
+    if (r >= M) return;
+    float ss = 0.f;
+#pragma unroll
+    for (int w = 0; w < kStepWarps; ++w) ss += ssq_part[w][r];
+    v *= 1.0f / sqrtf(ss / (float)K + eps);
+    if (c >= E) {
+        z[(int64_t)r * E + (c - E)] = __float2bfloat16_rn(v);
+        return;
+    }
+    // conv step on the bf16-rounded in_proj output, as the unfused path sees it
+    const float xc = __bfloat162float(__float2bfloat16_rn(v));
+    __nv_bfloat16 *st = conv_state + (int64_t)r * 3 * E + c;
+    const float x0 = __bfloat162float(st[0]), x1 = __bfloat162float(st[E]), x2 = __bfloat162float(st[2 * E]);
+    float wt[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int src = j - (4 - Kc);
+        wt[j] = src >= 0 ? cw[(int64_t)c * Kc + src] : 0.f;
+    }
+    float cv = cb ? cb[c] : 0.f;
+    cv += wt[0] * x0;
+    cv += wt[1] * x1;
+    cv += wt[2] * x2;
+    cv += wt[3] * xc;
+    u[(int64_t)r * E + c] = __float2bfloat16_rn(silu_acc(cv));
+    st[0] = __float2bfloat16_rn(x1);
+    st[E] = __float2bfloat16_rn(x2);
+    st[2 * E] = __float2bfloat16_rn(xc);
+}
+
+template <int MT>
+__global__ void __launch_bounds__(kStepWarps * 32)
+inproj_step_kernel(const float *__restrict__ resid, const float *__restrict__ norm_w, float eps,
+                   const __nv_bfloat16 *__restrict__ W, __nv_bfloat16 *__restrict__ conv_state,
+                   const float *__restrict__ cw, const float *__restrict__ cb, __nv_bfloat16 *__restrict__ u,
+                   __nv_bfloat16 *__restrict__ z, int M, int K, int E, int Kc) {
+    inproj_step_body<MT, false>(resid, norm_w, eps, W, conv_state, cw, cb, u, z, M, K, E, Kc);
+}
+template <int MT>
+__global__ void __launch_bounds__(kStepWarps * 32)
+inproj_step_chain_kernel(const float *resid, const float *__restrict__ norm_w, float eps, const __nv_bfloat16 *__restrict__ W,
+                         __nv_bfloat16 *conv_state, const float *__restrict__ cw, const float *__restrict__ cb, __nv_bfloat16 *u,
+                         __nv_bfloat16 *z, int M, int K, int E, int Kc) {
+    inproj_step_body<MT, true>(resid, norm_w, eps, W, conv_state, cw, cb, u, z, M, K, E, Kc);
+}
+
+// The same for a chain (launch_chained) of at most kAheadK columns, and for 17 to 32 rows: 8 warps (with 16 a CTA takes so many
+// registers that the 384 CTAs of a 768-wide model do not fit the device at once) request the weights of their first three
+// k-blocks, all there are, before chain_wait().  A wider K would take a second trip, in which the order of its loads costs more
+// than the first one hides: one row, us, this kernel / the one above: K = 1024 6.8 / 5.0, 2048 13.5 / 9.8.
 // A CTA takes 8 * NT columns.  Every CTA reads and scales the whole residual stream [M, K], which for one or two rows of
-// 16 costs nothing, but for 32 rows was most of the kernel (384 CTAs x 98 KB through L2, 8.9 us): 16 columns then.
-// The weights of a warp's first kStepPre k-blocks (all of them up to K = 768) are requested before chain_wait().
-constexpr int kStepPre = 3;
+// 16 costs nothing, but for 32 rows was most of the kernel (384 CTAs x 98 KB through L2, 8.9 us): 16 columns then, as long as
+// every SM still gets a CTA ([32, 512]: 128 CTAs of 16 columns 4.6 us, 256 of 8 3.9 us).  More than 32 rows take it where there
+// are few CTAs or two waves of them (a step, us, this kernel / the one above: [64, 128] 11.1 / 12.5, [64, 768] 30.2 / 33.8, but
+// [33, 512] 18.0 / 15.5, [64, 512] 21.3 / 20.1, [33, 1024] 33.4 / 31.4).
+constexpr int kAheadWarps = 8, kAheadBlocks = 3, kAheadK = kAheadWarps * kAheadBlocks * 32;
 
 template <int MT, int NT>
-__global__ void __launch_bounds__(kStepWarps * 32, MT == 1 ? 3 : MT == 2 ? 2 : 1)
-inproj_step_kernel(const float *resid, const float *__restrict__ norm_w, float eps, const __nv_bfloat16 *__restrict__ W,
-                   __nv_bfloat16 *conv_state, const float *__restrict__ cw, const float *__restrict__ cb, __nv_bfloat16 *u,
-                   __nv_bfloat16 *z, int M, int K, int E, int Kc, int prefetch) {
-    __shared__ float partial[kStepWarps * MT * NT * 128];
-    __shared__ float ssq_part[kStepWarps][MT * 16];
+__global__ void __launch_bounds__(kAheadWarps * 32, MT == 1 ? 3 : MT == 2 ? 2 : 1)
+inproj_step_ahead_kernel(const float *resid, const float *__restrict__ norm_w, float eps, const __nv_bfloat16 *__restrict__ W,
+                         __nv_bfloat16 *conv_state, const float *__restrict__ cw, const float *__restrict__ cb, __nv_bfloat16 *u,
+                         __nv_bfloat16 *z, int M, int K, int E, int Kc) {
+    __shared__ float partial[kAheadWarps * MT * NT * 128];
+    __shared__ float ssq_part[kAheadWarps][MT * 16];
     chain_trigger();
-    if (!prefetch) chain_wait();   // the kernel before this one may write weights
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tid = lane & 3;
     const int n0 = blockIdx.x * 8 * NT;
@@ -178,12 +310,12 @@ inproj_step_kernel(const float *resid, const float *__restrict__ norm_w, float e
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.f;
     }
-    uint4 b[kStepPre][NT];
-    float4 w0[kStepPre], w1[kStepPre];
+    uint4 b[kAheadBlocks][NT];
+    float4 w0[kAheadBlocks], w1[kAheadBlocks];
     auto fetch_w = [&](int k0) {
 #pragma unroll
-        for (int p = 0; p < kStepPre; ++p) {
-            const int k = k0 + p * kStepWarps * 32;
+        for (int p = 0; p < kAheadBlocks; ++p) {
+            const int k = k0 + p * kAheadWarps * 32;
             if (k >= K) break;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)   // n0 + nt * 8 + g < 2E: the W row this lane loads (2E is a multiple of 8 * NT)
@@ -194,12 +326,12 @@ inproj_step_kernel(const float *resid, const float *__restrict__ norm_w, float e
     };
     fetch_w(warp * 32);
     // outputs this thread finishes: which row and column, and what the conv step of that column needs
-    constexpr int OUTS = MT * NT * 128, PER = (OUTS + kStepWarps * 32 - 1) / (kStepWarps * 32);
+    constexpr int OUTS = MT * NT * 128, PER = (OUTS + kAheadWarps * 32 - 1) / (kAheadWarps * 32);
     int orow[PER], ocol[PER];
     float wt[PER][4], cbias[PER], xs[PER][3];
 #pragma unroll
     for (int o = 0; o < PER; ++o) {
-        const int t = threadIdx.x + o * kStepWarps * 32;
+        const int t = threadIdx.x + o * kAheadWarps * 32;
         const int mt = t / (NT * 128), nt = (t >> 7) % NT, ln = (t & 127) >> 2, i = t & 3;
         orow[o] = mt * 16 + (i >> 1) * 8 + (ln >> 2);
         ocol[o] = n0 + nt * 8 + 2 * (ln & 3) + (i & 1);
@@ -220,11 +352,11 @@ inproj_step_kernel(const float *resid, const float *__restrict__ norm_w, float e
         for (int j = 0; j < 3; ++j)
             xs[o][j] = conv ? __bfloat162float(conv_state[((int64_t)orow[o] * 3 + j) * E + ocol[o]]) : 0.f;
     }
-    for (int k0 = warp * 32; k0 < K; k0 += kStepPre * kStepWarps * 32) {
+    for (int k0 = warp * 32; k0 < K; k0 += kAheadBlocks * kAheadWarps * 32) {
         if (k0 != warp * 32) fetch_w(k0);
 #pragma unroll
-        for (int p = 0; p < kStepPre; ++p) {
-            const int k = k0 + p * kStepWarps * 32;
+        for (int p = 0; p < kAheadBlocks; ++p) {
+            const int k = k0 + p * kAheadWarps * 32;
             if (k >= K) break;   // warp-uniform
             uint4 a[MT][2];
 #pragma unroll
@@ -282,11 +414,11 @@ inproj_step_kernel(const float *resid, const float *__restrict__ norm_w, float e
     __syncthreads();
 #pragma unroll
     for (int o = 0; o < PER; ++o) {
-        const int t = threadIdx.x + o * kStepWarps * 32, r = orow[o], c = ocol[o];
+        const int t = threadIdx.x + o * kAheadWarps * 32, r = orow[o], c = ocol[o];
         if (r >= M) continue;
         float v = 0.f, ss = 0.f;
 #pragma unroll
-        for (int w = 0; w < kStepWarps; ++w) {
+        for (int w = 0; w < kAheadWarps; ++w) {
             v += partial[w * OUTS + t];
             ss += ssq_part[w][r];
         }
@@ -413,15 +545,28 @@ hx_status hx::mamba_block_step(const hx_mamba_step_args *a, bool chained, void *
     int64_t z_stride = 2 * E;
     if (fused) {
         auto zp = static_cast<__nv_bfloat16 *>(xz);  // the xz area holds z [B, E] here
-#define HX_INPROJ_STEP(MT, NT)                                                                                       \
-        HX_CUDA(hx::launch_chained(chained, inproj_step_kernel<MT, NT>, dim3((unsigned)(2 * E / (8 * NT))), dim3(kStepWarps * 32), \
-                                   st, a->residual, a->norm_w, a->norm_eps, static_cast<const __nv_bfloat16 *>(a->W_in), \
+#define HX_INPROJ_STEP(KERNEL, COLS, WARPS)                                                                          \
+        HX_CUDA(hx::launch_chained(chained, KERNEL, dim3((unsigned)(2 * E / (COLS))), dim3((WARPS) * 32), st, a->residual, a->norm_w, \
+                                   a->norm_eps, static_cast<const __nv_bfloat16 *>(a->W_in),                         \
                                    static_cast<__nv_bfloat16 *>(a->conv_state), a->conv_w, a->conv_b,                \
-                                   static_cast<__nv_bfloat16 *>(u), zp, Bn, M, E, a->d_conv, chained ? 1 : 0))
-        if (Bn <= 16) HX_INPROJ_STEP(1, 1);
-        else if (Bn <= 32 && E % 8 == 0) HX_INPROJ_STEP(2, 2);
-        else if (Bn <= 32) HX_INPROJ_STEP(2, 1);
-        else HX_INPROJ_STEP(4, 1);
+                                   static_cast<__nv_bfloat16 *>(u), zp, Bn, M, E, a->d_conv))
+#define HX_INPROJ_STEP_ROWS(MT)                                                                                      \
+        if (chained) HX_INPROJ_STEP(inproj_step_chain_kernel<MT>, 8, kStepWarps);                                    \
+        else HX_INPROJ_STEP(inproj_step_kernel<MT>, 8, kStepWarps)
+        if (chained && Bn <= 16 && M <= kAheadK) {
+            HX_INPROJ_STEP((inproj_step_ahead_kernel<1, 1>), 8, kAheadWarps);
+        } else if (Bn > 16 && Bn <= 32 && E % 8 == 0 && 2 * E / 16 >= hx::sm_count()) {
+            HX_INPROJ_STEP((inproj_step_ahead_kernel<2, 2>), 16, kAheadWarps);
+        } else if (Bn > 32 && (M <= 128 || (Bn > 48 && M >= 768))) {
+            HX_INPROJ_STEP((inproj_step_ahead_kernel<4, 1>), 8, kAheadWarps);
+        } else if (Bn <= 16) {
+            HX_INPROJ_STEP_ROWS(1);
+        } else if (Bn <= 32) {
+            HX_INPROJ_STEP_ROWS(2);
+        } else {
+            HX_INPROJ_STEP_ROWS(4);
+        }
+#undef HX_INPROJ_STEP_ROWS
 #undef HX_INPROJ_STEP
         if ((s = hx::check_launch("inproj_step_kernel")) != HX_OK) return s;
         z_bf = zp;

@@ -77,36 +77,31 @@ gemm_skinny_body(const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16 *W, in
             for (int h = 0; h < 2; ++h) a[mt][h] = (a_ok[mt][h] && k < K) ? *reinterpret_cast<const uint4 *>(arow[mt][h] + k) : zero4;
     };
     uint4 a[2][MT][2];
-    if constexpr (!CHAIN) {  // two blocks per trip so that their loads overlap
-        for (int k0 = warp * 32; k0 < K; k0 += 2 * STEP) {
-            uint4 b[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                b[u] = ld_w(k0 + u * STEP);
-                ld_a(a[u], k0 + u * STEP);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) mma(a[u], b[u]);
-        }
-    } else {                 // four of W, the first trip's before the wait, and twice two of A
+    int k0 = warp * 32;
+    if constexpr (CHAIN) {  // four blocks of W before the wait, then twice two of A
         uint4 b[4];
-        auto fetch_w = [&](int k0) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) b[u] = ld_w(k0 + u * STEP);
-        };
-        fetch_w(warp * 32);
+        for (int u = 0; u < 4; ++u) b[u] = ld_w(k0 + u * STEP);
         chain_wait();
-        for (int k0 = warp * 32; k0 < K; k0 += 4 * STEP) {
-            if (k0 != warp * 32) fetch_w(k0);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (k0 + half * 2 * STEP >= K) break;   // warp-uniform
+        for (int half = 0; half < 2; ++half) {
+            if (k0 >= K) break;   // warp-uniform
 #pragma unroll
-                for (int u = 0; u < 2; ++u) ld_a(a[u], k0 + (half * 2 + u) * STEP);
+            for (int u = 0; u < 2; ++u) ld_a(a[u], k0 + u * STEP);
 #pragma unroll
-                for (int u = 0; u < 2; ++u) mma(a[u], b[half * 2 + u]);
-            }
+            for (int u = 0; u < 2; ++u) mma(a[u], b[half * 2 + u]);
+            k0 += 2 * STEP;
         }
+    }
+    for (; k0 < K; k0 += 2 * STEP) {  // two blocks per trip so that their loads overlap
+        uint4 b[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            b[u] = ld_w(k0 + u * STEP);
+            ld_a(a[u], k0 + u * STEP);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) mma(a[u], b[u]);
     }
     // partial[warp][mt][lane][i]; accumulator layout: i = 0, 1 -> (row g, columns 2 tid, 2 tid + 1); i = 2, 3 -> row g + 8
 #pragma unroll
