@@ -53,7 +53,6 @@ conv_silu_kernel(const T *__restrict__ x, int64_t xb, int64_t xr, const float *_
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int d = g * VN;
     if (d >= D) return;
-    const int t0 = blockIdx.y * TB;
     const int b = blockIdx.z;
     float w[VN][4], bias[VN];
 #pragma unroll
@@ -72,67 +71,71 @@ conv_silu_kernel(const T *__restrict__ x, int64_t xb, int64_t xr, const float *_
     }
     const T *xp = x + b * xb + d;
     T *up = u + b * ub + d;
-    float win[3][VN];  // x[t-3], x[t-2], x[t-1]
+    // a grid holds 65 535 strips in this direction; a longer sequence takes further rounds
+    for (int64_t ts = (int64_t)blockIdx.y * TB; ts < L; ts += (int64_t)gridDim.y * TB) {
+        const int t0 = (int)ts;
+        float win[3][VN];  // x[t-3], x[t-2], x[t-1]
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const int t = t0 - 3 + j;
-        if (t >= 0) {
+        for (int j = 0; j < 3; ++j) {
+            const int t = t0 - 3 + j;
+            if (t >= 0) {
+                if constexpr (VEC) {
+                    Vec<T> v;
+                    v.load(xp + t * xr);
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) win[j][e] = v.v[e];
+                } else {
+                    win[j][0] = ld_f32(xp + t * xr);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < VN; ++e) win[j][e] = 0.f;
+            }
+        }
+        float rows[TB][VN];  // every row of the strip is requested before the first one is used
+#pragma unroll
+        for (int k = 0; k < TB; ++k) {
+            const int t = t0 + k;
+            if (t < L) {
+                if constexpr (VEC) {
+                    Vec<T> v;
+                    v.load(xp + t * xr);
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) rows[k][e] = v.v[e];
+                } else {
+                    rows[k][0] = ld_f32(xp + t * xr);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < VN; ++e) rows[k][e] = 0.f;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TB; ++k) {
+            const int t = t0 + k;
+            if (t >= L) break;
+            float out[VN];
+            const float (&cur)[VN] = rows[k];
+#pragma unroll
+            for (int e = 0; e < VN; ++e) {
+                float c = bias[e];
+                c += w[e][0] * win[0][e];
+                c += w[e][1] * win[1][e];
+                c += w[e][2] * win[2][e];
+                c += w[e][3] * cur[e];
+                out[e] = FASTM ? silu_fast(c) : silu_acc(c);
+                win[0][e] = win[1][e];
+                win[1][e] = win[2][e];
+                win[2][e] = cur[e];
+            }
             if constexpr (VEC) {
                 Vec<T> v;
-                v.load(xp + t * xr);
 #pragma unroll
-                for (int e = 0; e < VN; ++e) win[j][e] = v.v[e];
+                for (int e = 0; e < VN; ++e) v.v[e] = out[e];
+                v.store(up + t * ur);
             } else {
-                win[j][0] = ld_f32(xp + t * xr);
+                st_f32(up + t * ur, out[0]);
             }
-        } else {
-#pragma unroll
-            for (int e = 0; e < VN; ++e) win[j][e] = 0.f;
-        }
-    }
-    float rows[TB][VN];  // every row of the strip is requested before the first one is used
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-        const int t = t0 + k;
-        if (t < L) {
-            if constexpr (VEC) {
-                Vec<T> v;
-                v.load(xp + t * xr);
-#pragma unroll
-                for (int e = 0; e < VN; ++e) rows[k][e] = v.v[e];
-            } else {
-                rows[k][0] = ld_f32(xp + t * xr);
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < VN; ++e) rows[k][e] = 0.f;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-        const int t = t0 + k;
-        if (t >= L) break;
-        float out[VN];
-        const float (&cur)[VN] = rows[k];
-#pragma unroll
-        for (int e = 0; e < VN; ++e) {
-            float c = bias[e];
-            c += w[e][0] * win[0][e];
-            c += w[e][1] * win[1][e];
-            c += w[e][2] * win[2][e];
-            c += w[e][3] * cur[e];
-            out[e] = FASTM ? silu_fast(c) : silu_acc(c);
-            win[0][e] = win[1][e];
-            win[1][e] = win[2][e];
-            win[2][e] = cur[e];
-        }
-        if constexpr (VEC) {
-            Vec<T> v;
-#pragma unroll
-            for (int e = 0; e < VN; ++e) v.v[e] = out[e];
-            v.store(up + t * ur);
-        } else {
-            st_f32(up + t * ur, out[0]);
         }
     }
 }
@@ -416,7 +419,8 @@ hx_status hx_conv1d_silu_fwd(const void *x, int64_t xb, int64_t xr, const float 
     const bool vec = d_inner % vn == 0 && xr % vn == 0 && ur % vn == 0 && xb % vn == 0 && ub % vn == 0 &&
                      (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0;
     const int groups = vec ? d_inner / vn : d_inner;
-    dim3 grid((groups + 63) / 64, (seq_len + TB - 1) / TB, batch), block(64);
+    const int strips = seq_len / TB + (seq_len % TB != 0);
+    dim3 grid((groups + 63) / 64, strips < 65535 ? strips : 65535, batch), block(64);
     if (io_dtype == HX_BF16) {
         auto fits = [&](int ch) {
             return d_inner % ch == 0 && xr % ch == 0 && ur % ch == 0 && xb % ch == 0 && ub % ch == 0 &&

@@ -85,6 +85,22 @@ def test_conv1d_silu(dtype, B, L, D, K):
         assert fp32_tol_err(to_np(got), ref) <= FP32_TOL
 
 
+@pytest.mark.parametrize("dtype,D", [("f32", 4), ("f32", 3), ("bf16", 3)])
+@pytest.mark.parametrize("L", [8 * 65535, 8 * 65535 + 9, 2097120])
+def test_conv1d_silu_long_sequences(dtype, D, L):
+    """Sequences of as many strips as a grid holds, of more, and the longest that strips of 32 steps took."""
+    import torch
+    from helixml_b200 import ops
+    x = to_dev(synth.round_bf16(synth.normal(41, "x", (1, L, D))), dtype if dtype == "bf16" else None)
+    w = to_dev(synth.normal(41, "w", (D, 4), 0, 0.5))
+    got = ops.conv1d_silu(x, w)
+    xd = torch.nn.functional.pad(x.double(), (0, 0, 3, 0))
+    c = sum(xd[:, j:j + L] * w.double()[:, j] for j in range(4))
+    ref = c * torch.sigmoid(c)
+    err = ((got.double() - ref).abs() / (1 + ref.abs())).max().item()
+    assert err <= (1e-2 if dtype == "bf16" else FP32_TOL), err
+
+
 @pytest.mark.parametrize("B,L,E,NO", [(1, 128, 64, 16), (2, 300, 128, 80), (1, 5, 64, 40), (3, 1000, 1536, 80), (1, 257, 256, 256),
                                       (2, 131, 192, 8), (20, 1000, 64, 24)])   # the last: enough tiles for the 128-step form
 def test_conv_silu_and_x_proj_in_one_kernel(B, L, E, NO):
