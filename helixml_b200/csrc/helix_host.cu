@@ -85,7 +85,8 @@ struct DeviceTensor::Storage {
     void *p = nullptr;
     int dev = 0;
     bool pooled = false;
-    std::atomic<bool> escaped{false};
+    std::atomic<bool> escaped{false};  // a caller has the address
+    std::atomic<bool> settled{false};  // and the work queued before it was asked for is complete
     ~Storage() {
         if (pooled && !escaped.load(std::memory_order_acquire)) hx::pool_release(p, dev);
         else hx::pool_discard(p, dev);
@@ -133,9 +134,32 @@ Result<DeviceTensor> DeviceTensor::pooled(const Shape &shape, DType dtype, const
     return t;
 }
 
+// Waits for the legacy default stream of `dev`.  The caller may be capturing a stream of its own, in which an ordinary wait is
+// a forbidden call that ends the capture: the wait is made in the relaxed mode, and left out (false) while a stream that is
+// ordered with the default stream is being captured.  The current device stays what it is.
+static bool wait_for_default_stream(int dev) {
+    int prev = -1;
+    if (cudaGetDevice(&prev) != cudaSuccess || (prev != dev && cudaSetDevice(dev) != cudaSuccess)) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool ok = cudaStreamIsCapturing(nullptr, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+                    cudaStreamSynchronize(nullptr) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (prev != dev) cudaSetDevice(prev);
+    return ok;
+}
+
 void *DeviceTensor::data_for_caller() const {
-    if (storage_ && storage_->pooled && !storage_->escaped.exchange(true, std::memory_order_acq_rel)) {
-        if (use_device(device_).ok()) cudaStreamSynchronize(nullptr);
+    if (storage_ && storage_->pooled) {
+        storage_->escaped.store(true, std::memory_order_release);
+        // every caller waits until one wait has succeeded: an address is not given out before the contents are there
+        if (!storage_->settled.load(std::memory_order_acquire) && wait_for_default_stream(storage_->dev))
+            storage_->settled.store(true, std::memory_order_release);
     }
     return ptr_;
 }

@@ -94,7 +94,7 @@ class DeviceTensor {
     static Result<DeviceTensor> pooled(const Shape &shape, DType dtype, const Device &device);
     static Result<DeviceTensor> zeros(const Shape &shape, DType dtype, const Device &device);
     // The address for code outside this library, which may use it on any stream: the work queued so far is complete
-    // when this returns, and the block goes back with cudaFree, which waits for every stream, instead of to the cache.
+    // when this returns (unless a stream ordered with the default stream is being captured), and the block goes back with cudaFree, which waits for every stream, instead of to the cache.
     void *data_for_caller() const;
     // host data is fp32 (or bytes for U8); it is converted to `dtype` on the way in
     static Result<DeviceTensor> from_host_f32(const float *data, const Shape &shape, DType dtype, const Device &device,

@@ -556,6 +556,31 @@ def test_byte_lm_captured_prefill_after_a_larger_profiled_one():
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+def test_address_of_a_result_inside_a_capture():
+    """Asking for a result's address, which waits for the work queued before it, leaves a capture of another stream intact,
+    and so does asking from a second thread; the address holds the finished result either way."""
+    import threading
+    import torch
+    from helixml_b200 import nn
+    src = np.arange(1 << 20, dtype=np.float32)
+    a, b = (nn.Tensor.from_numpy(src).mul_scalar(k) for k in (2.0, 3.0))
+    x = torch.ones(8, device="cuda")
+    torch.cuda.synchronize()
+    ptr = {}
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x += 1
+        ptr["a"] = a.data_ptr()
+        t = threading.Thread(target=lambda: ptr.setdefault("b", b.data_ptr()))
+        t.start()
+        t.join()
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.all(x == 3) and ptr["a"] and ptr["b"] and ptr["a"] != ptr["b"]
+    assert a.data_ptr() == ptr["a"] and np.array_equal(a.numpy(), src * 2) and np.array_equal(b.numpy(), src * 3)
+
+
 def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
     """A result's memory returns to the block cache and the next result of its size is correct; an address handed to the
     caller keeps its contents while other results come and go."""
