@@ -40,8 +40,9 @@ struct Pool {
     std::unordered_map<void *, size_t> size_of;        // every block of this device, cached or in use
     size_t cached = 0;
 };
+// Never destroyed: a tensor may be released by a destructor that runs after this file's at process exit.
 Pool *pool_of(int dev) {
-    static Pool pools[64];
+    static Pool *pools = new Pool[64];
     return dev >= 0 && dev < 64 ? &pools[dev] : nullptr;
 }
 // small sizes in steps of 512 bytes, large ones in steps of 1/8 of their power of two: the shapes of one workload

@@ -581,6 +581,29 @@ def test_address_of_a_result_inside_a_capture():
     assert a.data_ptr() == ptr["a"] and np.array_equal(a.numpy(), src * 2) and np.array_equal(b.numpy(), src * 3)
 
 
+def test_result_released_after_the_library_at_exit(tmp_path):
+    """A result that is still held when the process exits, released by a destructor that runs after the library's own
+    static objects are gone: the process ends normally."""
+    import subprocess
+    import sys
+    from helixml_b200 import _lib
+    src = tmp_path / "late.c"
+    src.write_text("#include <stdlib.h>\nstatic void *held; static void (*drop)(void *);\n"
+                   "void hold(void *t, void (*f)(void *)) { held = t; drop = f; }\n"
+                   "__attribute__((destructor)) static void late(void) { if (drop) drop(held); }\n")
+    so = tmp_path / "late.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", str(src), "-o", str(so)], check=True)
+    prog = ("import ctypes as C, sys, numpy as np\n"
+            f"late = C.CDLL({str(so)!r})\n"
+            "from helixml_b200 import nn, _lib\n"
+            "ts = [nn.Tensor.from_numpy(np.ones(n, np.float32)).add_scalar(1.0) for n in range(1000, 1400)]\n"
+            "assert ts[7].numpy()[0] == 2\n"
+            "late.hold(ts[7]._h, C.cast(_lib.lib().hx_tensor_free, C.c_void_p))\n"
+            "ts[7]._h = None\n")
+    r = subprocess.run([sys.executable, "-c", prog], cwd=_lib.__file__.rsplit("/", 2)[0], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
+
+
 def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
     """A result's memory returns to the block cache and the next result of its size is correct; an address handed to the
     caller keeps its contents while other results come and go."""
