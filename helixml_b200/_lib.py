@@ -92,6 +92,7 @@ _PROTOS = {
     "hx_set_device": (C.c_int, [C.c_int]),
     "hx_alloc": (C.c_int, [C.POINTER(C.c_void_p), C.c_size_t]),
     "hx_free": (C.c_int, [C.c_void_p]),
+    "hx_memory_trim": (C.c_int, [C.c_int32]),
     "hx_host_alloc": (C.c_int, [C.POINTER(C.c_void_p), C.c_size_t]),
     "hx_host_free": (C.c_int, [C.c_void_p]),
     "hx_memcpy_h2d": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),

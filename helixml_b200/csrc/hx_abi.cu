@@ -64,11 +64,10 @@ struct OnDevice {  // makes `dev` current for a scope
 };
 }  // namespace
 
-void pool_trim() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
+void pool_trim(int dev) {
     Pool *p = pool_of(dev);
     if (!p) return;
+    OnDevice scope(dev);
     std::lock_guard<std::mutex> lock(p->mu);
     for (auto &b : p->free_blocks) {
         p->size_of.erase(b.second);
@@ -167,6 +166,14 @@ hx_status hx_set_device(int device) {
     return HX_OK;
 }
 
+hx_status hx_memory_trim(int32_t device_id) {
+    int n = 0;
+    HX_CUDA(cudaGetDeviceCount(&n));
+    HX_REQUIRE(device_id >= 0 && device_id < n, HX_ERR_INVALID_INPUT, "device %d of %d", device_id, n);
+    hx::pool_trim(device_id);
+    return HX_OK;
+}
+
 hx_status hx_alloc(void **dptr, size_t bytes) {
     HX_REQUIRE(dptr != nullptr, HX_ERR_INVALID_INPUT, "hx_alloc: dptr is NULL");
     *dptr = nullptr;
@@ -174,7 +181,8 @@ hx_status hx_alloc(void **dptr, size_t bytes) {
     cudaError_t e = cudaMalloc(dptr, bytes);
     if (e == cudaErrorMemoryAllocation) {  // the memory may be in the module layer's block cache
         cudaGetLastError();
-        hx::pool_trim();
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess) hx::pool_trim(dev);
         e = cudaMalloc(dptr, bytes);
     }
     if (e != cudaSuccess) {

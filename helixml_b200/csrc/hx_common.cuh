@@ -52,7 +52,7 @@ constexpr size_t kPoolCachedBytes = (size_t)512 << 20;
 hx_status pool_alloc(void **dptr, size_t bytes);
 void pool_release(void *dptr, int device);   // back to the cache; `device` is where it was allocated
 void pool_discard(void *dptr, int device);   // a real cudaFree (waits for the device)
-void pool_trim();                            // gives every cached block of the current device back
+void pool_trim(int device);                  // gives every cached block of the device back
 
 // resid[i] += x[i] (x fp32 or bf16): the residual update where no GEMM epilogue can do it.
 hx_status residual_add(float *resid, const void *x, int x_dtype, int64_t n, cudaStream_t st);

@@ -294,6 +294,11 @@ class Module:
             pass
 
 
+def trim_memory(device: Device = Device(0)) -> None:
+    """Gives the device memory that released results left in the module layer's cache back (hx_memory_trim)."""
+    L.check(L.lib().hx_memory_trim(device.index))
+
+
 def manual_seed(seed: int) -> None:
     L.lib().hx_manual_seed(C.c_uint64(seed))
 

@@ -87,6 +87,9 @@ HX_API hx_status hx_device_count(int *count);
 HX_API hx_status hx_set_device(int device);
 HX_API hx_status hx_alloc(void **dptr, size_t bytes);
 HX_API hx_status hx_free(void *dptr);
+/* The module layer keeps up to 512 MiB of released result and workspace blocks per device for its next calls.  This gives
+ * them back (cudaFree, which waits for the device); an allocation of this library that fails does so by itself. */
+HX_API hx_status hx_memory_trim(int32_t device_id);
 HX_API hx_status hx_host_alloc(void **hptr, size_t bytes);   /* pinned host memory */
 HX_API hx_status hx_host_free(void *hptr);
 HX_API hx_status hx_memcpy_h2d(void *dst, const void *src_host, size_t bytes, void *stream);

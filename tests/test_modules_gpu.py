@@ -605,8 +605,8 @@ def test_result_released_after_the_library_at_exit(tmp_path):
 
 
 def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
-    """A result's memory returns to the block cache and the next result of its size is correct; an address handed to the
-    caller keeps its contents while other results come and go."""
+    """A result's memory returns to the block cache, the next result of its size takes it and is correct, and trim_memory
+    gives it back; an address handed to the caller keeps its contents while other results come and go."""
     import torch
     from helixml_b200 import nn
     a = np.arange(12345, dtype=np.float32)
@@ -615,5 +615,17 @@ def test_result_blocks_are_reused_and_caller_addresses_stay_valid():
     for i in range(20):
         t = nn.Tensor.from_numpy(a * i)
         assert np.array_equal(t.mul_scalar(2.0).numpy(), a * i * 2)
+    big = np.ones(16 << 20, dtype=np.float32)  # 64 MiB
+    nn.trim_memory()
+    free = lambda: torch.cuda.mem_get_info()[0]
+    before = free()
+    for i in range(12):
+        t = nn.Tensor.from_numpy(big).mul_scalar(2.0)
+    del t
+    torch.cuda.synchronize()
+    held = before - free()
+    assert (64 << 20) <= held <= 4 * (64 << 20), held  # cached, and not a block per result
+    nn.trim_memory()
+    assert before - free() < 64 << 20
     torch.cuda.synchronize()
     assert np.array_equal(kept.numpy(), a + 1)
