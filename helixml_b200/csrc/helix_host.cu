@@ -769,51 +769,62 @@ Result<Unit> ByteLM::parameters_updated() {
     return Unit{};
 }
 
-// Makes the activation buffers hold (batch, seq_len).  They only ever grow, by at least half of what they are: prompts of
-// changing length run in the same memory (allocating per shape cost 1 to 100 ms a prompt, and every captured forward with
-// it, since cudaFree waits for the device).  Captured forwards point into these buffers and into the decode state, so
-// both functions drop them before they replace any of it: no caller has to.
+// A call keeps what earlier, larger calls left allocated unless that is more than four times its need and more than this.
+static constexpr size_t kHeldBytes = (size_t)1 << 30;
+static bool holds_too_much(int64_t need, int64_t cap, size_t unit_bytes) {
+    return need < cap / 4 && (size_t)cap * unit_bytes > kHeldBytes;
+}
+
+// Activation buffers for n tokens in place of those there are; the workspace stays.
+Result<Unit> ByteLM::alloc_activations(int64_t n) {
+    drop_forwards();
+    if (!buf_) buf_ = new Buffers();
+    buf_->tokens_cap = 0;
+    buf_->tokens = buf_->resid = buf_->normed = buf_->block_out = buf_->logits = DeviceTensor();
+    HELIX_ASSIGN(buf_->tokens, DeviceTensor::empty(Shape({n}), DType::U8, device_));
+    HELIX_ASSIGN(buf_->resid, DeviceTensor::empty(Shape({n, d_model}), DType::F32, device_));
+    HELIX_ASSIGN(buf_->normed, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
+    HELIX_ASSIGN(buf_->block_out, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
+    HELIX_ASSIGN(buf_->logits, DeviceTensor::empty(Shape({n, 256}), dtype, device_));
+    buf_->tokens_cap = n;
+    return Unit{};
+}
+
+Result<Unit> ByteLM::alloc_workspace(size_t bytes) {
+    drop_forwards();
+    buf_->workspace_cap = 0;
+    buf_->workspace = DeviceTensor();
+    HELIX_ASSIGN(buf_->workspace, DeviceTensor::empty(Shape({(int64_t)bytes}), DType::U8, device_));
+    buf_->workspace_cap = bytes;
+    return Unit{};
+}
+
+// Makes the activation buffers hold (batch, seq_len).  They grow by at least half of what they are and are kept for smaller
+// calls: prompts of changing length run in the same memory (allocating per shape cost 1 to 100 ms a prompt, and every
+// captured forward with it, since cudaFree waits for the device).  Captured forwards point into these buffers and into the
+// decode state, so whatever replaces any of it drops them first: no caller has to.
 Result<Unit> ByteLM::ensure_buffers(int64_t batch, int64_t seq_len) {
     const int64_t T = batch * seq_len;
-    if (!buf_) buf_ = new Buffers();
-    if (T > buf_->tokens_cap) {
-        drop_forwards();
-        const int64_t grown = buf_->tokens_cap + buf_->tokens_cap / 2;
-        const int64_t cap = T > grown ? T : grown;
-        delete buf_;
-        buf_ = new Buffers();
-        auto fill = [&](int64_t n) -> Result<Unit> {
-            HELIX_ASSIGN(buf_->tokens, DeviceTensor::empty(Shape({n}), DType::U8, device_));
-            HELIX_ASSIGN(buf_->resid, DeviceTensor::empty(Shape({n, d_model}), DType::F32, device_));
-            HELIX_ASSIGN(buf_->normed, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
-            HELIX_ASSIGN(buf_->block_out, DeviceTensor::empty(Shape({n, d_model}), dtype, device_));
-            HELIX_ASSIGN(buf_->logits, DeviceTensor::empty(Shape({n, 256}), dtype, device_));
-            buf_->tokens_cap = n;
-            return Unit{};
-        };
-        auto r = fill(cap);
-        if (!r.ok() && cap > T) {  // no room for the spare half
-            delete buf_;
-            buf_ = new Buffers();
-            r = fill(T);
-        }
+    const size_t token_bytes = 1 + (size_t)d_model * 4 + (2 * (size_t)d_model + 256) * dtype_size(dtype);
+    const int64_t have = buf_ ? buf_->tokens_cap : 0;
+    const size_t wb = blocks[0]->workspace_bytes(batch, seq_len);
+    const bool shrink = buf_ && (holds_too_much(T, have, token_bytes) || holds_too_much((int64_t)wb, (int64_t)buf_->workspace_cap, 1));
+    if (T > have || shrink) {
+        if (shrink) buf_->workspace = DeviceTensor(), buf_->workspace_cap = 0;
+        const int64_t cap = shrink ? T : std::max(T, have + have / 2);
+        auto r = alloc_activations(cap);
+        if (!r.ok() && cap > T) r = alloc_activations(T);  // no room for the spare half
         if (!r.ok()) {
             delete buf_;
             buf_ = nullptr;
             return r.error();
         }
     }
-    const size_t wb = blocks[0]->workspace_bytes(batch, seq_len);
     if (wb > buf_->workspace_cap) {
-        drop_forwards();
         const size_t cap = std::max(wb, buf_->workspace_cap + buf_->workspace_cap / 2);
-        buf_->workspace_cap = 0;
-        buf_->workspace = DeviceTensor();
-        auto w = DeviceTensor::empty(Shape({(int64_t)cap}), DType::U8, device_);
-        if (!w.ok() && cap > wb) w = DeviceTensor::empty(Shape({(int64_t)wb}), DType::U8, device_);
-        if (!w.ok()) return w.error();
-        buf_->workspace = std::move(w.value());
-        buf_->workspace_cap = (size_t)buf_->workspace.numel();
+        auto r = alloc_workspace(cap);
+        if (!r.ok() && cap > wb) r = alloc_workspace(wb);
+        if (!r.ok()) return r.error();
     }
     buf_->batch = batch;
     buf_->seq_len = seq_len;
@@ -839,12 +850,7 @@ Result<Unit> ByteLM::prefill_device(const uint8_t *tokens_dev, void *logits_dev,
     return run_layers(tokens_dev, logits_dev, batch, seq_len, stream, true);
 }
 
-// The decode state of `batch` sequences.  The buffers grow only.
-Result<Unit> ByteLM::ensure_decode(int64_t batch) {
-    if (dec_ && dec_->cap >= batch) {
-        dec_->batch = batch;
-        return Unit{};
-    }
+Result<Unit> ByteLM::alloc_decode(int64_t batch) {
     drop_forwards();
     delete dec_;
     dec_ = new Decode();
@@ -865,6 +871,33 @@ Result<Unit> ByteLM::ensure_decode(int64_t batch) {
     dec_->batch = batch;
     dec_->cap = batch;
     return Unit{};
+}
+
+// The decode state of `batch` sequences, kept for smaller batches like the activation buffers.
+Result<Unit> ByteLM::ensure_decode(int64_t batch) {
+    const MambaBlock &b0 = *blocks[0];
+    const size_t row_bytes = blocks.size() * (size_t)b0.d_inner * ((size_t)b0.d_state * 4 + 3 * dtype_size(dtype));
+    if (dec_ && dec_->cap >= batch && !holds_too_much(batch, dec_->cap, row_bytes)) {
+        dec_->batch = batch;
+        return Unit{};
+    }
+    auto r = alloc_decode(batch);
+    if (!r.ok() && buf_) {  // the memory may be what the activation buffers hold beyond this call's shape
+        const int64_t T = buf_->batch * buf_->seq_len;
+        const size_t wb = b0.workspace_bytes(buf_->batch, buf_->seq_len);
+        if (buf_->tokens_cap > T || buf_->workspace_cap > wb) {
+            delete dec_;
+            dec_ = nullptr;
+            HELIX_TRY(alloc_workspace(wb));
+            HELIX_TRY(alloc_activations(T));
+            r = alloc_decode(batch);
+        }
+    }
+    if (!r.ok()) {
+        delete dec_;
+        dec_ = nullptr;
+    }
+    return r;
 }
 
 // One step over the module's own buffers (dec_->tokens in, dec_->logits out): what the graph captures.

@@ -299,6 +299,9 @@ class ByteLM : public Module {
   private:
     Result<Unit> ensure_buffers(int64_t batch, int64_t seq_len);
     Result<Unit> ensure_decode(int64_t batch);
+    Result<Unit> alloc_activations(int64_t tokens);
+    Result<Unit> alloc_workspace(size_t bytes);
+    Result<Unit> alloc_decode(int64_t batch);
     void drop_forwards();
     Result<Unit> enqueue_step(void *stream);
     Result<Unit> run_layers(const uint8_t *tokens_dev, void *logits_dev, int64_t batch, int64_t seq_len, void *stream,

@@ -556,6 +556,42 @@ def test_byte_lm_captured_prefill_after_a_larger_profiled_one():
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+def test_byte_lm_gives_back_what_a_small_call_does_not_need():
+    """After a call that needed gigabytes, one of a few tokens gives most of them back (activations, workspace and decode
+    state) and computes what a fresh model does."""
+    import torch
+    from helixml_b200 import nn
+    emb, layers, normf = _lm_weights(24, 2, 256)
+    tok = torch.from_numpy(synth.random_bytes(24, "t", (3, 50))).cuda()
+    nxt = torch.from_numpy(synth.random_bytes(24, "n", (3,))).cuda()
+    out = torch.empty(3, 50, 256, device="cuda", dtype=torch.bfloat16)
+    lg = torch.empty(3, 256, device="cuda", dtype=torch.bfloat16)
+
+    def small(lm):
+        lm.prefill_device(tok.data_ptr(), out.data_ptr(), 3, 50)
+        lm.decode_step_device(nxt.data_ptr(), lg.data_ptr(), 3)
+        torch.cuda.synchronize()
+        return out.clone(), lg.clone()
+
+    lm, fresh = nn.ByteLM(2, 256), nn.ByteLM(2, 256)
+    for m in (lm, fresh):
+        m.load_weights(emb, layers, normf)
+    want = small(fresh)
+    many = torch.zeros(20000, 32, device="cuda", dtype=torch.uint8)
+    big = torch.empty(20000 * 32, 256, device="cuda", dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    free = lambda: torch.cuda.mem_get_info()[0]
+    at_first = free()
+    lm.prefill_device(many.data_ptr(), big.data_ptr(), 20000, 32)
+    torch.cuda.synchronize()
+    held = at_first - free()
+    assert held > 5 << 30, held
+    for _ in range(3):
+        got = small(lm)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert at_first - free() < 1 << 30, at_first - free()
+
+
 def test_address_of_a_result_inside_a_capture():
     """Asking for a result's address, which waits for the work queued before it, leaves a capture of another stream intact,
     and so does asking from a second thread; the address holds the finished result either way."""
