@@ -82,32 +82,17 @@ __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.l
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... V>
-inline cudaError_t launch_chained_smem(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster,
-                                       cudaStream_t st, V... args) {
+inline cudaError_t launch_chained(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, V... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    int n = 0;
-    if (chain) {
-        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[n++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster > 1) {
-        at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = cluster;
-        at[n].val.clusterDim.y = 1;
-        at[n++].val.clusterDim.z = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = n;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = chain ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-template <typename... P, typename... V>
-inline cudaError_t launch_chained(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, V... args) {
-    return launch_chained_smem(chain, kernel, grid, block, 0, 1, st, args...);
 }
 
 // hx_mamba_block_step; `chained`: the kernel queued before this call on `stream` is part of the same decode step, so
