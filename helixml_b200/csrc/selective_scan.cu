@@ -5,8 +5,8 @@
 // Two kernels:
 //   scan_simple_kernel  one thread per (batch, channel), any d_state <= 256, accurate libm-style
 //                       math.  The parity baseline (HX_SCAN_SIMPLE).
-//                       HX_SCAN_AUTO runs scan_wide_kernel (scan_wide.cu) for the shapes the other
-//                       kernels do not take.
+//                       HX_SCAN_AUTO runs scan_wide_kernel (scan_wide.cu), or this one where the chains
+//                       are plentiful, for the shapes the other kernels do not take.
 //   scan_tiled_kernel   d_state == 16.  A CTA owns one batch row and a 128-byte-wide channel tile
 //                       and walks the sequence in chunks.  A producer warp moves [chunk x tile]
 //                       boxes of x/dt/z/B/C into shared memory with TMA (3-D tensor maps, 128-byte
@@ -1209,6 +1209,11 @@ ScanKind auto_kind(const hx_scan_args *a) {
     return ScanKind::Tiled;
 }
 
+// Between the two general kernels: with chains enough for 20 warps of them per SM and bf16 operands, one thread per channel
+// is ahead up to 16 states (us, one thread / states over lanes: [64, 256, 2048] 4 states 616 / 928, [128, 128, 4096] 12 states 1271 /
+// 2042, but [32, 512, 1536], 10 warps per SM, 1082 / 775); with fp32 operands it never is ([128, 128, 4096] 4 states 1344 / 869).
+bool states_fit_a_thread(const hx_scan_args *a) { return a->io_dtype == HX_BF16 && a->d_state <= 16 && warps_per_sm(a) >= 20.0; }
+
 // Sequence segments for AUTO.
 int auto_splits(const hx_scan_args *a) {
     if (auto_looks_back(a)) {
@@ -1272,7 +1277,7 @@ hx_status hx_selective_scan_fwd(const hx_scan_args *a, void *stream) {
                 // an operand that does not meet the TMA alignment rules goes to the general kernel
                 if (s != HX_ERR_UNSUPPORTED_OPERATION) return s;
             }
-            return hx::scan::launch_wide(a, st);
+            return hx::scan::states_fit_a_thread(a) ? hx::scan::launch_simple(a, st) : hx::scan::launch_wide(a, st);
         }
         default: return hx::fail(HX_ERR_INVALID_INPUT, "unknown scan variant %d", a->variant);
     }

@@ -76,6 +76,16 @@ def test_wide_kernel(dtype, d_state, seq_len, d_inner):
           run_ref(inp, gate=False, skip=False, conv=False, softplus=False), dtype)
 
 
+@pytest.mark.parametrize("d_state,d_inner", [(1, 4096), (12, 4097), (16, 4099), (17, 4096)])
+def test_general_kernels_with_many_chains(d_state, d_inner):
+    """bf16 calls of 20 and more warps of chains per SM: one thread per channel up to 16 states, states over lanes past that."""
+    inp = synth.scan_inputs(72, 24, 9, d_inner, d_state, 4, bf16=True)
+    got, hg = run_gpu(inp, "bf16", variant=0, geom=False, state=True)
+    ref, hr = run_ref(inp, state=True)
+    check(got, ref, "bf16")
+    assert fp32_tol_err(hg, hr) <= FP32_TOL
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_simple_kernel(dtype):
     inp = synth.scan_inputs(31, 2, 50, 40, 16, 4, bf16=dtype == "bf16")
