@@ -181,15 +181,21 @@ static hx_status launch_simt_cfg(const TA *a, int64_t lda, const TA *w, int64_t 
 
 // The largest tile that still gives three quarters of the SMs one each: a bigger tile does more products per operand
 // read, but an idle SM costs more than that.  The smallest tiles split the inner dimension four ways inside the CTA.
+// Up to 64 columns half or more of a big tile would be padding: 64 x 64 tiles with slabs of 16 there (100000 x 16 x 16 9.7 us
+// against 17.0, 65536 x 64 x 64 17.7 against 31, 65536 x 64 x 1024 251 against 423); where the middle tile is the choice it stays
+// ahead of them (8000 x 64 x 4096 209 against 273).
 template <typename TA, typename TC, bool VEC>
 static hx_status launch_simt_tiles(const TA *a, int64_t lda, const TA *w, int64_t ldw, const float *bias, TC *c, int64_t ldc,
                                    int M, int N, int K, int epi, cudaStream_t st) {
     using Big = SimtCfg<128, 128, 8, 8, 1, 8>;
     using Mid = SimtCfg<64, 64, 8, 8, 4, 8>;
     using Small = SimtCfg<32, 32, 4, 4, 4, 16>;
+    using Narrow = SimtCfg<64, 64, 4, 4, 1, 16>;
     auto tiles = [&](int bm, int bn) { return (int64_t)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
     const int64_t enough = (int64_t)sm_count() * 3 / 4;
-    if (tiles(Big::BM, Big::BN) >= enough) return launch_simt_cfg<TA, TC, Big, VEC>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi, st);
+    if (tiles(Big::BM, Big::BN) >= enough)
+        return N <= 64 ? launch_simt_cfg<TA, TC, Narrow, VEC>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi, st)
+                       : launch_simt_cfg<TA, TC, Big, VEC>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi, st);
     if (tiles(Mid::BM, Mid::BN) >= enough) return launch_simt_cfg<TA, TC, Mid, VEC>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi, st);
     return launch_simt_cfg<TA, TC, Small, VEC>(a, lda, w, ldw, bias, c, ldc, M, N, K, epi, st);
 }

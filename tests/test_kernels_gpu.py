@@ -219,7 +219,7 @@ def test_gemm_tcgen05_tile_widths(M, N, K):
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("M,N,K", [(31, 33, 61), (33, 31, 64), (32, 32, 130), (700, 641, 35), (641, 700, 36), (1500, 1400, 9),
-                                   (1409, 1536, 24)])
+                                   (1409, 1536, 24), (14209, 64, 16), (14300, 1, 20), (14273, 63, 17), (7105, 65, 33)])
 def test_gemm_simt_tiles(dtype, M, N, K):
     """Every tile size of the CUDA-core GEMM (by the number of tiles the shape has), ragged edges, an inner dimension that is
     not a multiple of four, and a C whose rows are not 16-byte aligned."""
