@@ -85,15 +85,12 @@ def ncu_traffic(workload, kernel):
 
 
 def scan_kernel_name(variant, cfg, splits=0):
-    """The kernel hx_selective_scan_fwd runs for this variant (HX_SCAN_AUTO: one lane per channel when there are at
-    least 8 warps of chains per SM, the lane-split kernel otherwise)."""
+    """The kernel hx_selective_scan_fwd runs for this variant; the library says which HX_SCAN_AUTO takes."""
     if variant == "auto":
         import torch
-        sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-        if cfg["batch"] * cfg["d_inner"] / 32.0 >= 8.0 * sms:
-            variant = "direct"
-        else:
-            variant = "lookback" if splits > 1 else "tiled"
+        from helixml_b200 import _lib, ops
+        kind = ops.auto_variant(cfg["batch"], cfg["seq_len"], cfg["d_inner"], torch.bfloat16, splits)
+        variant = {_lib.SCAN_DIRECT: "direct", _lib.SCAN_LOOKBACK: "lookback"}.get(kind, "tiled")
     return {"direct": "scan_direct_kernel", "simple": "scan_simple_kernel",
             "lookback": "scan_direct_kernel (look-back: aggregate pass + output pass)"}.get(variant, "scan_tiled_kernel")
 

@@ -102,6 +102,7 @@ _PROTOS = {
     "hx_selective_scan_fwd": (C.c_int, [C.POINTER(ScanArgs), C.c_void_p]),
     "hx_selective_scan_workspace_bytes": (C.c_int, [C.POINTER(ScanArgs), C.POINTER(C.c_size_t)]),
     "hx_selective_scan_suggest_splits": (C.c_int32, [C.POINTER(ScanArgs)]),
+    "hx_selective_scan_auto_variant": (C.c_int32, [C.POINTER(ScanArgs)]),
     "hx_selective_scan_host": (C.c_int, [C.POINTER(ScanArgs), C.c_void_p, C.c_size_t, C.c_void_p]),
     "hx_selective_scan_host_workspace_bytes": (C.c_int, [C.POINTER(ScanArgs), C.POINTER(C.c_size_t)]),
     "hx_selective_scan_fwd_noalloc": (C.c_int, [C.POINTER(ScanArgs), C.c_void_p]),

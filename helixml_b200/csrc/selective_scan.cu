@@ -1288,6 +1288,15 @@ int32_t hx_selective_scan_suggest_splits(const hx_scan_args *a) {
     return hx::scan::auto_splits(a);
 }
 
+int32_t hx_selective_scan_auto_variant(const hx_scan_args *a) {
+    if (!a || a->d_state != 16) return HX_SCAN_AUTO;
+    switch (hx::scan::auto_kind(a)) {
+        case hx::scan::ScanKind::Direct: return HX_SCAN_DIRECT;
+        case hx::scan::ScanKind::LookBack: return HX_SCAN_LOOKBACK;
+        default: return HX_SCAN_TILED;
+    }
+}
+
 hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *a, size_t *bytes) {
     HX_REQUIRE(a && bytes, HX_ERR_INVALID_INPUT, "hx_selective_scan_workspace_bytes: NULL argument");
     *bytes = 0;

@@ -80,6 +80,15 @@ def suggest_splits(batch, seq_len, d_inner, dtype, a_geometric=True) -> int:
     return int(L.lib().hx_selective_scan_suggest_splits(C.byref(a)))
 
 
+def auto_variant(batch, seq_len, d_inner, dtype, seq_splits=0, a_geometric=True) -> int:
+    """hx_selective_scan_auto_variant: what HX_SCAN_AUTO runs for a scan with softplus of this shape."""
+    a = L.ScanArgs()
+    a.batch, a.seq_len, a.d_inner, a.d_state = batch, seq_len, d_inner, 16
+    a.io_dtype = L.HX_BF16 if dtype == torch.bfloat16 else L.HX_F32
+    a.a_geometric, a.dt_softplus, a.seq_splits = (1 if a_geometric else 0), 1, seq_splits
+    return int(L.lib().hx_selective_scan_auto_variant(C.byref(a)))
+
+
 def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, conv_w=None, conv_b=None, dt_bias=None, dt_softplus=True,
                    variant=L.SCAN_AUTO, a_geometric=None, lanes_per_channel=0, return_state=False, out=None,
                    workspace=None, seq_splits=0, tune=0, dt_low=None, W_dt=None, z_is_gate=False):

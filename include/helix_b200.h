@@ -172,6 +172,10 @@ HX_API hx_status hx_selective_scan_workspace_bytes(const hx_scan_args *args, siz
  * on the current device: chained segments that even out the load when chains are plentiful, parallel segments
  * (look-back form) when they are few.  Pass it as args->seq_splits with a workspace. */
 HX_API int32_t hx_selective_scan_suggest_splits(const hx_scan_args *args);
+/* The variant whose kernel HX_SCAN_AUTO runs for these arguments (dimensions, types, flags and seq_splits; operands that
+ * miss the alignment rules go to a general kernel instead): HX_SCAN_DIRECT, HX_SCAN_LOOKBACK (two launches) or HX_SCAN_TILED
+ * for d_state 16, HX_SCAN_AUTO for the general kernels of any other. */
+HX_API int32_t hx_selective_scan_auto_variant(const hx_scan_args *args);
 /* The same operation on HOST activations: x, dt, z, Bm, Cm are read from (preferably pinned) host memory
  * with the strides given in args, staged into `dev_workspace` (caller-owned device memory of
  * hx_selective_scan_host_workspace_bytes() bytes), scanned, and y is copied back to the host pointer

@@ -8,6 +8,21 @@ import sys
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
+def test_scan_kernel_is_named_by_the_library():
+    """The stand-alone scan of 16 x 4096 x 1536 has 5 warps of chains per SM: one pass, one launch, also in segments; a shard of
+    an eighth of it looks back."""
+    import torch
+    sys.path.insert(0, ROOT)
+    import bench
+    from helixml_b200 import ops
+    cfg = {"batch": 16, "seq_len": 4096, "d_inner": 1536}
+    splits = ops.suggest_splits(16, 4096, 1536, torch.bfloat16)
+    assert splits > 1 and bench.scan_kernel_name("auto", cfg, splits) == "scan_direct_kernel"
+    assert bench.scan_kernel_name("auto", cfg, 1) == "scan_direct_kernel"
+    assert "look-back" in bench.scan_kernel_name("auto", dict(cfg, batch=2), ops.suggest_splits(2, 4096, 1536, torch.bfloat16))
+    assert bench.scan_kernel_name("tiled", cfg) == "scan_tiled_kernel" and "look-back" in bench.scan_kernel_name("lookback", cfg, 8)
+
+
 def test_reference_arm_prints_one_contract_line():
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1", "--warmup", "0"],
                          cwd=ROOT, capture_output=True, text=True, timeout=600)
