@@ -498,6 +498,23 @@ def test_mamba_block_bf16(B, L, M):
     assert rel_l2(to_np(got), ref) <= BF16_TOL
 
 
+@pytest.mark.parametrize("dtype,B,L,M", [("bf16", 2, 700, 320), ("bf16", 1, 513, 576), ("bf16", 3, 100, 192), ("f32", 2, 300, 96),
+                                         ("f32", 1, 600, 160)])
+def test_mamba_block_odd_dt_rank(dtype, B, L, M):
+    """dt_rank = ceil(d_model / 16) not a multiple of 8 (20, 36, 12; f32 6, 10): the x_proj row misses the alignment the fused
+    kernels want, and conv, x_proj, the dt projection and the scan run on the general ones."""
+    from helixml_b200 import ops
+    w = synth.mamba_block_weights(5, M, 16, 4, 2)
+    x = synth.normal(5, "x", (B, L, M))
+    big = ("W_in", "W_x", "W_dt", "W_out") if dtype == "bf16" else ()
+    w = {k: (synth.round_bf16(v) if k in big else v) for k, v in w.items()}
+    x = synth.round_bf16(x) if dtype == "bf16" else x
+    got = ops.mamba_block(to_dev(x, dtype if big else None), {k: to_dev(v, "bf16" if k in big else None) for k, v in w.items()}, 16, 4)
+    _status_ok()
+    ref = cbind.mamba_block(x, w, 16, 4)
+    assert rel_l2(to_np(got), ref) <= BF16_TOL if big else fp32_tol_err(to_np(got), ref) <= FP32_TOL
+
+
 def test_mamba_block_bf16_direct_scan_with_fused_dt():
     """The block with the one-lane-per-channel scan forced: the dt projection then runs inside the scan kernel."""
     from helixml_b200 import _lib, ops

@@ -76,6 +76,32 @@ def test_wide_kernel(dtype, d_state, seq_len, d_inner):
           run_ref(inp, gate=False, skip=False, conv=False, softplus=False), dtype)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("d_state,d_inner", [(8, 33), (16, 31), (64, 24), (128, 9)])
+def test_wide_kernel_views_and_results_over_an_operand(dtype, d_state, d_inner):
+    """x, z and y as columns of wider rows, B and C as slices of one row at odd offsets, and y written over x, dt or z."""
+    import torch
+    from helixml_b200 import _lib, ops
+    inp = synth.scan_inputs(73, 2, 41, d_inner, d_state, 4, bf16=dtype == "bf16")
+    cast = "bf16" if dtype == "bf16" else None
+    ref = run_ref(inp)
+    t = {k: to_dev(inp[k], cast if k in ("x", "dt", "z", "B", "C") else None) for k in ("x", "dt", "z", "B", "C", "A", "D", "conv_w")}
+    xz = torch.cat([t["x"], t["z"][..., :1], t["z"]], -1)
+    bc = torch.cat([t["B"][..., :3], t["B"], t["C"]], -1)
+    y = torch.full((2, 41, 2 * d_inner + 1), 7.0, dtype=t["x"].dtype, device="cuda")
+    out = y[..., 1:d_inner + 1]
+    args = lambda x, dt: (x, dt, t["A"], bc[..., 3:3 + d_state], bc[..., 3 + d_state:])
+    ops.selective_scan(*args(xz[..., :d_inner], t["dt"]), D=t["D"], z=xz[..., d_inner + 1:], conv_w=t["conv_w"], out=out,
+                       a_geometric=False)
+    check(to_np(out), ref, dtype)
+    assert bool((y[..., 0] == 7).all()) and bool((y[..., d_inner + 1:] == 7).all())
+    for over in ("x", "dt", "z"):
+        c = {k: t[k].clone() for k in ("x", "dt", "z")}
+        ops.selective_scan(*args(c["x"], c["dt"]), D=t["D"], z=c["z"], conv_w=t["conv_w"], out=c[over], a_geometric=False)
+        check(to_np(c[over]), ref, dtype)
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("d_state,d_inner", [(1, 4096), (12, 4097), (16, 4099), (17, 4096)])
 def test_general_kernels_with_many_chains(d_state, d_inner):
     """bf16 calls of 20 and more warps of chains per SM: one thread per channel up to 16 states, states over lanes past that."""
