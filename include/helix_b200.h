@@ -138,8 +138,10 @@ typedef struct hx_scan_args {
                                  `workspace`).  HX_SCAN_TILED / DIRECT: in order, each starting from its
                                  predecessor's final state, which evens out the load when batch * d_inner / tile
                                  is not a multiple of the SM slots.  HX_SCAN_LOOKBACK: at the same time.
-                                 HX_SCAN_AUTO: chained when chains are plentiful, look-back (for any A) when they are
-                                 few.  HX_SCAN_SEQSPLIT / LOOKBACK: 0 = four segments */
+                                 HX_SCAN_AUTO: chained when chains are plentiful, look-back (for any A, where dt_softplus
+                                 or a_geometric = 1 is set) when they are few.  HX_SCAN_SEQSPLIT / LOOKBACK: 0 = four
+                                 segments.  In the look-back form an infinite input may come out as NaN where the
+                                 others give an infinity */
     int32_t a_geometric;      /* 1: the caller asserts A[d][n] == (n+1) * A[d][0] (checked once with
                                  hx_scan_check_geometric); then exp(dt*A[d][n]) is evaluated as a power of
                                  exp(dt*A[d][0]), one exp per point instead of d_state.  0: a general A.  2: not known to
