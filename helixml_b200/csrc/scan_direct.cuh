@@ -131,8 +131,7 @@ struct DirectCfg {
 };
 
 // 2^x of a decay: bf16 I/O takes the special-function unit's form (2^-22 relative, subnormal results flushed to zero), fp32
-// I/O keeps exp2f.  With the former an fp32 scan is 0.1 to 0.5 % further from 64 bits (3 x 1111 x 640, general A: 2.022e-7
-// against 2.011e-7).
+// I/O keeps exp2f, whose results reach down through the subnormals.  (Scans without such decays measure the same with both.)
 template <bool FAST> __device__ __forceinline__ float decay_exp2(float x) { return FAST ? ex2_approx(x) : exp2f(x); }
 
 // The decay of a whole segment as the fold applies it to the state h.  Step by step, a zero state stays zero and an infinite
@@ -793,7 +792,9 @@ scan_direct_body(const CUtensorMap &tm_x, const CUtensorMap &tm_dt, const CUtens
                 }
                 if constexpr (AGG) continue;
                 const float2 ys = add2(acc[0], acc[1]);
-                yout[e] = (ys.x + ys.y + ds_[e] * u) * g;
+                // fp32 I/O: the gate is multiplied in by the last fma, as the lane-split kernel does it, one rounding less
+                if constexpr (FAST) yout[e] = (ys.x + ys.y + ds_[e] * u) * g;
+                else yout[e] = fmaf(ys.x + ys.y, g, ds_[e] * u * g);
             }
             if constexpr (AGG) return;
             // y goes straight from registers to HBM: the warp writes one contiguous run of 32*CPL channels

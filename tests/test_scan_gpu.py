@@ -613,6 +613,37 @@ def test_workspace_sized_for_chained_segments_serves_auto():
 
 
 @pytest.mark.parametrize("geom", [True, False])
+def test_fp32_forms_are_equally_far_from_64_bits(geom):
+    """The one-lane-per-channel and the lane-split kernel round the same number of times on the way to y: their distances
+    from 64 bits, over a million outputs, are within 0.3 % (0.1 % measured; 0.5 % with the gate as a rounding of its own)."""
+    import torch
+    from helixml_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(74)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    B, L, D = 8, 300, 512
+    x, z, Bm, Cm = rnd(B, L, D), rnd(B, L, D), rnd(B, L, 16), rnd(B, L, 16)
+    dt = torch.rand(B, L, D, device="cuda", generator=g) * 3 - 4
+    A = -torch.arange(1, 17, device="cuda", dtype=torch.float32).repeat(D, 1)
+    if not geom:
+        A = A * torch.exp(0.2 * rnd(D, 16))
+    skip, w = torch.ones(D, device="cuda"), torch.rand(D, 4, device="cuda", generator=g) - 0.5
+    d = lambda t: t.double()
+    xp = torch.nn.functional.pad(d(x), (0, 0, 3, 0))
+    u = torch.nn.functional.silu(sum(d(w)[:, j] * xp[:, j:j + L] for j in range(4)))
+    dtv = torch.nn.functional.softplus(d(dt), threshold=60)
+    h, ref = torch.zeros(B, D, 16, device="cuda", dtype=torch.float64), torch.empty_like(u)
+    for t in range(L):
+        h = torch.exp(dtv[:, t, :, None] * d(A)) * h + (dtv[:, t] * u[:, t])[..., None] * d(Bm)[:, t, None]
+        ref[:, t] = (h * d(Cm)[:, t, None]).sum(-1)
+    ref = (ref + u) * torch.nn.functional.silu(d(z))
+    err = {}
+    for v in (TILED, DIRECT):
+        y = ops.selective_scan(x, dt, A, Bm, Cm, D=skip, z=z, conv_w=w, variant=v, a_geometric=geom)
+        err[v] = ((d(y) - ref).norm() / ref.norm()).item()
+    assert err[DIRECT] <= 1.003 * err[TILED], err
+
+
+@pytest.mark.parametrize("geom", [True, False])
 @pytest.mark.parametrize("variant,splits,step", [(DIRECT, 0, 1.0), (TILED, 0, 1.0), (0, 3, 1.0 / 16)])
 def test_fp32_decays_keep_subnormal_results(geom, variant, splits, step):
     """Decays of 1e-41 to 6e-39 (subnormal) times a state of 1e37: per step (one pass) and over a 16-step segment (the
